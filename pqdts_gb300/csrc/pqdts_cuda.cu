@@ -2262,34 +2262,40 @@ static void run_stage(Ctx& c, int mode, int oiter, int maxiiter, double conv_thr
   c.timers.flush();
 }
 
-static void get_x_colmajor(Ctx& c, double* out) {
-  const int64_t M = c.h.M, N = c.h.N;
-  std::vector<double> rm((size_t)M * N);
-  CK(cudaMemcpyAsync(rm.data(), c.X.p, rm.size() * 8, cudaMemcpyDeviceToHost, c.st));
+// X-shaped arrays across the ABI are (M, N) column-major, on the device
+// row-major: they are copied as they are and transposed on the device.  The
+// staging copy is entry `slot` of the line-search candidates' stack, whose
+// contents outlive a line search only up to the update that adopts one of
+// them (outer_tail), never an entry point.
+template <typename T>
+static void upload_colmajor(Ctx& c, const double* in, T* dev, int slot = 0) {
+  const int M = (int)c.h.M, N = (int)c.h.N;
+  const int64_t MN = (int64_t)M * N;
+  double* stage = c.Xc.p + slot * MN;
+  CK(cudaMemcpyAsync(stage, in, MN * sizeof(double), cudaMemcpyHostToDevice, c.st));
+  k_transpose<double, T><<<cdiv(M, 32) * cdiv(N, 32), 256, 0, c.st>>>(stage, N, M, dev);
+  post_launch(c);
+}
+
+template <typename T>
+static void download_colmajor(Ctx& c, const T* dev, double* out) {
+  const int M = (int)c.h.M, N = (int)c.h.N;
+  k_transpose<T, double><<<cdiv(M, 32) * cdiv(N, 32), 256, 0, c.st>>>(dev, M, N, c.Xc.p);
+  post_launch(c);
+  CK(cudaMemcpyAsync(out, c.Xc.p, (int64_t)M * N * sizeof(double), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
-  c.d2h += (int64_t)rm.size() * 8;
-  for (int64_t i = 0; i < M; ++i)
-    for (int64_t n = 0; n < N; ++n) out[i + n * M] = rm[(size_t)i * N + n];
+}
+
+static void get_x_colmajor(Ctx& c, double* out) {
+  download_colmajor(c, c.X.p, out);
+  c.d2h += c.h.M * c.h.N * 8;
 }
 
 static void set_x_colmajor(Ctx& c, const double* in) {
-  const int64_t M = c.h.M, N = c.h.N;
-  std::vector<double> rm((size_t)M * N);
-  for (int64_t i = 0; i < M; ++i)
-    for (int64_t n = 0; n < N; ++n) rm[(size_t)i * N + n] = in[i + n * M];
-  CK(cudaMemcpyAsync(c.X.p, rm.data(), rm.size() * 8, cudaMemcpyHostToDevice, c.st));
+  upload_colmajor(c, in, c.X.p);
   CK(cudaStreamSynchronize(c.st));
-  c.h2d += (int64_t)rm.size() * 8;
+  c.h2d += c.h.M * c.h.N * 8;
   touch_x(c);
-}
-
-static void download_rowmajor_to_col(Ctx& c, const double* dev, double* out) {
-  const int64_t M = c.h.M, N = c.h.N;
-  std::vector<double> rm((size_t)M * N);
-  CK(cudaMemcpyAsync(rm.data(), dev, rm.size() * 8, cudaMemcpyDeviceToHost, c.st));
-  CK(cudaStreamSynchronize(c.st));
-  for (int64_t i = 0; i < M; ++i)
-    for (int64_t n = 0; n < N; ++n) out[i + n * M] = rm[(size_t)i * N + n];
 }
 
 static void fill_stats(Ctx& c, const SolveState& st, double secs, double* stats) {
@@ -3121,7 +3127,7 @@ int pqdts_cuda_dL(pqdts_ctx* c, double* G) {
   return guarded(c, [&] {
     pqdts::need_problem(*c);
     pqdts::op_dL(*c);
-    pqdts::download_rowmajor_to_col(*c, c->G.p, G);
+    pqdts::download_colmajor(*c, c->G.p, G);
   });
 }
 
@@ -3142,18 +3148,15 @@ int pqdts_cuda_BF(pqdts_ctx* c, const double* V, double* HV) {
   return guarded(c, [&] {
     pqdts::need_problem(*c);
     const int64_t M = c->h.M, N = c->h.N;
-    std::vector<double> rm((size_t)M * N);
-    for (int64_t i = 0; i < M; ++i)
-      for (int64_t n = 0; n < N; ++n) rm[(size_t)i * N + n] = V[i + n * M];
     auto& b = c->cg64;
-    CK(cudaMemcpyAsync(b.p.p, rm.data(), rm.size() * 8, cudaMemcpyHostToDevice, c->st));
+    pqdts::upload_colmajor(*c, V, b.p.p);
     if (!c->fullspace) {
       pqdts::k_cg_lift<double><<<pqdts::cdiv(M, 32), pqdts::kLiftThreads, 0, c->st>>>(
           nullptr, 0, (int)M, (int)N, b.p.p, b.z.p, c->maxr.p, b.V.p, b.rs.p);
       pqdts::post_launch(*c);
     }
     pqdts::hvp<double>(*c, b, c->fval.p, c->tval.p, nullptr, false);
-    pqdts::download_rowmajor_to_col(*c, b.Hp.p, HV);
+    pqdts::download_colmajor(*c, b.Hp.p, HV);
   });
 }
 
@@ -3162,40 +3165,28 @@ int pqdts_cuda_BF32(pqdts_ctx* c, const double* V, double* HV) {
     pqdts::need_problem(*c);
     if (c->precision != PQDTS_MIXED) throw Err(PQDTS_E_STATE, "BF32 needs a mixed-precision problem");
     const int64_t M = c->h.M, N = c->h.N;
-    std::vector<float> rm((size_t)M * N);
-    for (int64_t i = 0; i < M; ++i)
-      for (int64_t n = 0; n < N; ++n) rm[(size_t)i * N + n] = (float)V[i + n * M];
     auto& b = c->cg32;
-    CK(cudaMemcpyAsync(b.p.p, rm.data(), rm.size() * 4, cudaMemcpyHostToDevice, c->st));
-    c->h2d += (int64_t)rm.size() * 4;
+    pqdts::upload_colmajor(*c, V, b.p.p);
+    c->h2d += M * N * 8;
     if (!c->fullspace) {
       pqdts::k_cg_lift32<<<pqdts::cdiv(M * 32, 256), 256, 0, c->st>>>(nullptr, 0, (int)M, (int)N, b.p.p, b.z.p,
                                                                      c->maxr.p, b.V.p, b.rs.p);
       pqdts::post_launch(*c);
     }
     pqdts::hvp32(*c, b, nullptr, false, nullptr);
-    CK(cudaMemcpyAsync(rm.data(), b.Hp.p, rm.size() * 4, cudaMemcpyDeviceToHost, c->st));
     pqdts::read_back(*c, c->sc.p, pqdts::SC_NSC);
     pqdts::check_tc_error(*c);
-    c->d2h += (int64_t)rm.size() * 4;
-    for (int64_t i = 0; i < M; ++i)
-      for (int64_t n = 0; n < N; ++n) HV[i + n * M] = rm[(size_t)i * N + n];
+    pqdts::download_colmajor(*c, b.Hp.p, HV);
+    c->d2h += M * N * 8;
   });
 }
 
 int pqdts_cuda_pdot(pqdts_ctx* c, const double* A, const double* B, double* out) {
   return guarded(c, [&] {
     pqdts::need_problem(*c);
-    const int64_t M = c->h.M, N = c->h.N;
-    std::vector<double> ra((size_t)M * N), rb((size_t)M * N);
-    for (int64_t i = 0; i < M; ++i)
-      for (int64_t n = 0; n < N; ++n) {
-        ra[(size_t)i * N + n] = A[i + n * M];
-        rb[(size_t)i * N + n] = B[i + n * M];
-      }
     auto& b = c->cg64;
-    CK(cudaMemcpyAsync(b.p.p, ra.data(), ra.size() * 8, cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(b.z.p, rb.data(), rb.size() * 8, cudaMemcpyHostToDevice, c->st));
+    pqdts::upload_colmajor(*c, A, b.p.p, 0);
+    pqdts::upload_colmajor(*c, B, b.z.p, 1);
     pqdts::dot_dev(*c, b.p.p, b.z.p, c->sc.p + pqdts::SC_TMP);
     CK(cudaMemcpyAsync(out, c->sc.p + pqdts::SC_TMP, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));

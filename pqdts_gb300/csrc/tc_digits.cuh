@@ -1,0 +1,453 @@
+// Banded products of FP64 operands on the tensor cores, by exact integer
+// digits: the mixed path's gradient F^T.R (dL, pqdts.f90:975-1032) and its
+// FP64-accurate objective checks F.X - P (L, 917-973).
+//
+// Every operand row of F (or F^T) and every column of X (or R) is scaled by
+// a power of two, so that its largest magnitude lies in [1/4, 1/2), rounded
+// to 48 bits and written as kDgS = 6 signed digits in base 256, each exact
+// in bf16:
+//   x = 2^E (d_0 2^-8 + d_1 2^-16 + ... + d_5 2^-48),  |d_q| <= 128.
+// A product is then a sum over digit pairs, and the pairs p + q = L of one
+// level L share a weight 2^(-8 (L + 2)), so level L needs one integer sum
+//   S_L = sum_k sum_{p + q = L} dF_p[k] dX_q[k]
+// which the MMAs (bf16 in, FP32 accumulator in tensor memory) form exactly:
+// a product of digits is at most 2^14, and the accumulators are drained into
+// 64-bit integers every kDgDrain = 8 chunks of K = 32, so a pair's sum stays
+// within 256 * 2^14 = 2^22 and the levels 0..3 within 2^24, the integers an
+// FP32 accumulator holds; levels 4 and 5 may pass that (by at most 1.5x,
+// operands whose digits all have one sign) and then round by an ulp, 2^-48
+// of the scales.  Levels 0..5 are kept (21 digit pairs): the error of a sum
+// is ~sqrt(K) 2^-47 of (row scale x column scale), measured against 64 bits
+// 2e-15 to 6e-15 of the result's norm where the double-FP32 kernels
+// (k_fwd_df, k_trans_df) are 1.3e-14 to 4e-14 off.
+//
+// This replaces ~12 FP32 operations a term on the CUDA cores by 21 bf16
+// MMA terms.  One CTA per SM walks a list of 128 x BN output tiles.  The
+// digits of a K chunk are one TMA box each: A 6 x 128 rows, B 6 x BN rows of
+// 64 bytes (64-byte swizzle), so with A's digit p the digits 0 .. 5 - p of B
+// are (6 - p) BN consecutive rows, and their products belong to the levels p
+// .. 5, consecutive column blocks of the accumulator: one MMA instruction
+// (or two, N <= 256) per digit of A instead of one per pair, which is what
+// keeps shared memory (A read 8 times a K slice instead of 21) below the
+// tensor pipe.  BN = 64 fills 384 of the 512 tensor-memory columns; a stage
+// is 72 KB and three fit.  The drain is not overlapped with the MMAs (no
+// room for a second accumulator), eight warps share it; the output of a
+// tile is formed and stored while the next tile's MMAs run.
+#pragma once
+
+#include "tc_band.cuh"
+
+namespace pqdts {
+
+constexpr int kDgS = 6;       // base-256 digits an operand
+constexpr int kDgDrain = 8;   // K chunks (of kTcK) between drains
+constexpr int kDgThreads = 320;  // TMA warp, MMA warp, 8 epilogue warps
+constexpr int kDgMaxStages = 4;
+constexpr uint32_t kDgRing = 216u * 1024u;
+
+// Biased exponent of a double's magnitude (2047: infinite or NaN).
+__device__ __forceinline__ int dg_exponent(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff); }
+
+// The kDgS digits (bf16 bit patterns, most significant first) of v, whose
+// biased exponent is at most emax: v = 2^(emax - 1069) t, t = v's mantissa
+// shifted to the scale's 48 bits, rounded half away from zero; each byte of
+// t + 0x808080808080 is a digit + 128.
+__device__ __forceinline__ void dg_digits(double v, int emax, uint32_t (&d)[kDgS]) {
+  const long long b = __double_as_longlong(v);
+  int e = (int)((b >> 52) & 0x7ff);
+  unsigned long long m = (unsigned long long)b & ((1ull << 52) - 1);
+  if (e != 0) m |= 1ull << 52;
+  else e = 1;
+  const int sh = max(emax, 1) - e + 6;  // >= 6
+  const unsigned long long t = sh <= 54 ? (m + (1ull << (sh - 1))) >> sh : 0ull;  // <= 2^47
+  const unsigned long long u = (b < 0 ? 0ull - t : t) + 0x808080808080ull;
+#pragma unroll
+  for (int q = 0; q < kDgS; ++q) {
+    const uint32_t byte = (uint32_t)(u >> (8 * (kDgS - 1 - q))) & (q == 0 ? 0x1ffu : 0xffu);
+    // 2^23 + byte as a float, minus 2^23 + 128: the digit, exactly
+    d[q] = __float_as_uint(__fsub_rn(__uint_as_float(0x4b000000u | byte), 8388736.0f)) >> 16;
+  }
+}
+
+// Largest biased exponent of each column of X (R x N row-major) into
+// colexp[n] (zeroed by the caller): block (32 columns) x (a share of the
+// rows, grid.y shares).
+__global__ void __launch_bounds__(256) k_dg_colexp(const double* __restrict__ X, int R, int N,
+                                                   int* __restrict__ colexp) {
+  __shared__ int s[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n = blockIdx.x * 32 + lane;
+  int e = 0;
+  if (n < N)
+    for (int r = blockIdx.y * 8 + w; r < R; r += gridDim.y * 8) e = max(e, dg_exponent(X[(int64_t)r * N + n]));
+  s[w][lane] = e;
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) e = max(e, s[q][lane]);
+    if (n < N && e > 0) atomicMax(colexp + n, e);
+  }
+}
+
+// Digits of X (R x N row-major) as the products' K-major operand: digit q of
+// X[r, n] at out[(q * N + n) * ld + r] (ld >= R, even).  A block transposes
+// 64 rows x 32 columns through shared memory; HBM bound (8 bytes in, 12 out).
+__global__ void __launch_bounds__(256) k_dg_split_t(const double* __restrict__ X, int R, int N,
+                                                    const int* __restrict__ colexp, int64_t ld,
+                                                    uint16_t* __restrict__ out) {
+  __shared__ __align__(4) uint16_t t[kDgS][32][66];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * 64, n0 = blockIdx.y * 32;
+  {
+    const int n = n0 + lane;
+    const int emax = n < N ? colexp[n] : 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int y = w + 8 * k, r = r0 + y;
+      const double v = (r < R && n < N) ? X[(int64_t)r * N + n] : 0.0;
+      uint32_t d[kDgS];
+      dg_digits(v, emax, d);
+#pragma unroll
+      for (int q = 0; q < kDgS; ++q) t[q][lane][y] = (uint16_t)d[q];
+    }
+  }
+  __syncthreads();
+  const int r = r0 + 2 * lane;
+#pragma unroll 4
+  for (int x = w; x < kDgS * 32; x += 8) {
+    const int q = x >> 5, n = n0 + (x & 31);
+    if (n >= N || r >= R) continue;
+    uint16_t* o = out + ((int64_t)q * N + n) * ld + r;
+    if (r + 1 < R) *reinterpret_cast<uint32_t*>(o) = *reinterpret_cast<const uint32_t*>(&t[q][x & 31][2 * lane]);
+    else *o = t[q][x & 31][2 * lane];
+  }
+}
+
+// Digits of the band operand: row r's values val[off .. off + w) at columns
+// lo .. lo + w - 1 of F (TRANS: of F^T, whose rows are contiguous in d) ->
+// digit q at out[(q * rows + r) * kmax + (column - kb[r / 128])], zero
+// elsewhere, and the row's exponent.  One block per padded row.
+template <bool TRANS>
+__global__ void __launch_bounds__(256) k_dg_band(DevBands f, const double* __restrict__ val,
+                                                 const int32_t* __restrict__ kb, int rows, int kmax,
+                                                 uint16_t* __restrict__ out, int* __restrict__ rowexp) {
+  __shared__ int s_e;
+  const int r = blockIdx.x, R = TRANS ? f.M : f.D;
+  int lo = 0, w = 0;
+  int64_t off = 0;
+  if (r < R) {
+    if (TRANS) {
+      off = f.tptr[r];
+      w = (int)(f.tptr[r + 1] - off);
+      if (w > 0) lo = f.tidx[off];
+    } else if (f.flo[r] >= 0) {
+      lo = f.flo[r];
+      w = f.fw[r];
+      off = f.foff[r];
+    }
+  }
+  if (threadIdx.x == 0) s_e = 0;
+  __syncthreads();
+  int e = 0;
+  for (int k = threadIdx.x; k < w; k += blockDim.x) e = max(e, dg_exponent(val[off + k]));
+  if (e > 0) atomicMax(&s_e, e);
+  __syncthreads();
+  e = s_e;
+  if (threadIdx.x == 0) rowexp[r] = e;
+  const int start = lo - max(kb[r / kTcRows], 0);  // first local column of the band
+  for (int x = threadIdx.x; x < kmax; x += blockDim.x) {
+    const int k = x - start;
+    const double v = (unsigned)k < (unsigned)w ? val[off + k] : 0.0;
+    uint32_t d[kDgS];
+    dg_digits(v, e, d);
+#pragma unroll
+    for (int q = 0; q < kDgS; ++q) out[((int64_t)q * rows + r) * kmax + x] = (uint16_t)d[q];
+  }
+}
+
+// 3-D TMA tile load (x, y, z = K, row, digit) completing on `bar`.
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+      "[%5];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// 8 consecutive columns of this thread's accumulator row in each of the six
+// levels (level stride `ls` columns), waited in place.
+__device__ __forceinline__ void dg_ld8x6(uint32_t a, uint32_t ls, float (&v)[kDgS][8]) {
+  uint32_t r[48];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%48];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%49];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%50];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%51];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%32, %33, %34, %35, %36, %37, %38, %39}, [%52];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%40, %41, %42, %43, %44, %45, %46, %47}, [%53];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]),
+        "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]),
+        "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47])
+      : "r"(a), "r"(a + ls), "r"(a + 2 * ls), "r"(a + 3 * ls), "r"(a + 4 * ls), "r"(a + 5 * ls)
+      : "memory");
+#pragma unroll
+  for (int q = 0; q < kDgS; ++q)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[q][j] = __uint_as_float(r[8 * q + j]);
+}
+
+// Operands and results of one digit product.
+struct DgArgs {
+  const int32_t *kb, *nch;           // K window of each 128-row block of A
+  const int *rowexp, *colexp;        // exponents of A's rows and B's columns
+  const int32_t *sched_off, *sched_tile;  // each CTA's tiles (N tile fastest, then row block)
+  int R, N, BN, stages;
+  // what the epilogue adds (MODE 0, 3: P; MODE 4: the gamma stencil on V)
+  const double* P;
+  const double* V;
+  double c2gam;
+  double *out, *out2;
+  // F itself and B's FP64 values, for columns that hold an infinity or a NaN
+  DevBands f;
+  const double *val, *B;
+  double* err;
+  uint64_t wait_ns;
+};
+
+// Row r of F (TRANS: F^T) times column n of B in plain FP64: the result for
+// a column with an infinite or NaN entry, which has no digits.
+template <bool TRANS>
+__device__ __noinline__ double dg_plain(const DgArgs& g, int r, int n) {
+  int lo = -1, w = 0;
+  int64_t off = 0;
+  if (TRANS) {
+    off = g.f.tptr[r];
+    w = (int)(g.f.tptr[r + 1] - off);
+    if (w > 0) lo = g.f.tidx[off];
+  } else if (g.f.flo[r] >= 0) {
+    lo = g.f.flo[r];
+    w = g.f.fw[r];
+    off = g.f.foff[r];
+  }
+  double s = 0.0;
+  for (int k = 0; k < w; ++k) s = fma(g.val[off + k], g.B[(int64_t)(lo + k) * g.N + n], s);
+  return s;
+}
+
+// MODE 0: out = 2 (F.B - P); MODE 3: out = F.B - P (R = D rows of F);
+// MODE 4: F^T.B + the gamma stencil on V into out and / or out2 (R = M rows
+// of F^T; either may be null).  Every wait is bounded as in k_tc_band; a
+// wait that runs out sets *err and the CTA stores nothing more, lets the
+// copies and MMAs in flight finish and frees its tensor memory.
+template <int MODE>
+__global__ void __launch_bounds__(kDgThreads, 1)
+    k_dg_band_product(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
+                      const __grid_constant__ DgArgs g) {
+  extern __shared__ uint8_t tc_smem_raw[];
+  __shared__ uint64_t bar_full[kDgMaxStages], bar_empty[kDgMaxStages], bar_accf, bar_acce, bar_fin;
+  __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_abort;
+  __shared__ int s_issued, s_consumed;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int BN = g.BN, N = g.N, stages = g.stages;
+  const int ntn = (N + BN - 1) / BN;
+  const uint32_t raw = smem_u32(tc_smem_raw);
+  uint8_t* base = tc_smem_raw + ((1024u - (raw & 1023u)) & 1023u);
+  const uint32_t a_slice = kTcRows * kTcRowBytes, b_slice = (uint32_t)BN * kTcRowBytes;
+  const uint32_t a_bytes = kDgS * a_slice, stage_bytes = a_bytes + kDgS * b_slice;
+  const uint32_t ncols = kDgS * BN <= 128 ? 128u : kDgS * BN <= 256 ? 256u : 512u;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&mA);
+    tma_prefetch_desc(&mB);
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(&bar_full[i], 1);
+      mbar_init(&bar_empty[i], 1);
+    }
+    mbar_init(&bar_accf, 1);
+    mbar_init(&bar_acce, 256);
+    mbar_init(&bar_fin, 1);
+    s_abort = 0;
+    s_issued = 0;
+    s_consumed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    tc_alloc(&s_tmem, ncols);
+    tc_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = s_tmem;
+  const int j_begin = g.sched_off[blockIdx.x], j_end = g.sched_off[blockIdx.x + 1];
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int j = j_begin; j < j_end && !s_abort; ++j) {
+        const int t = g.sched_tile[j], nt = t % ntn, blk = t / ntn, kb = g.kb[blk];
+        const int nk = kb >= 0 ? g.nch[blk] : 0;
+        for (int ch = 0; ch < nk && !s_abort; ++ch, ++it) {
+          const int st = it % stages;
+          const uint32_t ph = (uint32_t)(it / stages) & 1u;
+          if (!mbar_wait(&bar_empty[st], ph ^ 1u, g.wait_ns)) {
+            s_abort = 1;
+            break;
+          }
+          uint8_t* sa = base + (size_t)st * stage_bytes;
+          mbar_expect_tx(&bar_full[st], stage_bytes);
+          tma_load_3d(sa, &mA, ch * kTcK, blk * kTcRows, 0, &bar_full[st]);
+          tma_load_3d(sa + a_bytes, &mB, kb + ch * kTcK, nt * BN, 0, &bar_full[st]);
+          s_issued = it + 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int it = 0;
+      uint32_t drain = 0;
+      for (int j = j_begin; j < j_end && !s_abort; ++j) {
+        const int blk = g.sched_tile[j] / ntn;
+        const int nk = g.kb[blk] >= 0 ? g.nch[blk] : 0;
+        for (int c0 = 0; c0 < nk && !s_abort; c0 += kDgDrain, ++drain) {
+          if (!mbar_wait(&bar_acce, (drain & 1u) ^ 1u, g.wait_ns)) {  // accumulator drained
+            s_abort = 1;
+            break;
+          }
+          tc_fence_after();
+          const int c1 = min(nk, c0 + kDgDrain);
+          for (int ch = c0; ch < c1; ++ch, ++it) {
+            const int st = it % stages;
+            const uint32_t ph = (uint32_t)(it / stages) & 1u;
+            if (!mbar_wait(&bar_full[st], ph, g.wait_ns)) {
+              s_abort = 1;
+              break;
+            }
+            s_consumed = it + 1;
+            tc_fence_after();
+            const uint32_t sa = smem_u32(base + (size_t)st * stage_bytes), sb = sa + a_bytes;
+#pragma unroll
+            for (int k = 0; k < kTcK / 16; ++k) {
+              const uint32_t o = 32u * k;
+#pragma unroll
+              for (int p = 0; p < kDgS; ++p) {
+                // A's digit p with B's digits 0 .. 5 - p: levels p .. 5.  The
+                // first product of a drain overwrites the accumulators: digit
+                // 0 of A does that for all levels.
+                const uint32_t acc0 = (ch > c0 || k > 0 || p > 0) ? 1u : 0u;
+                const int cols = (kDgS - p) * BN;
+                const uint64_t da = swz_desc(sa + (uint32_t)p * a_slice + o);
+                for (int c = 0; c < cols; c += 256) {
+                  const int n = min(256, cols - c);
+                  tc_mma(tmem + (uint32_t)(p * BN + c), da, swz_desc(sb + (uint32_t)c * kTcRowBytes + o),
+                         tc_idesc_bf16(kTcRows, n), acc0);
+                }
+              }
+            }
+            tc_commit(&bar_empty[st]);
+          }
+          tc_commit(&bar_accf);
+        }
+      }
+      tc_commit(&bar_fin);  // arrives once every MMA this CTA issued is done (aborted or not)
+    }
+  } else {
+    // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (rows of
+    // the tile), and one half of the N tile's columns
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int hc = BN >> 1;  // columns per half: 8 .. 32
+    uint32_t drain = 0;
+    bool ok = true;
+    for (int j = j_begin; j < j_end && ok; ++j) {
+      const int t = g.sched_tile[j], nt = t % ntn, blk = t / ntn;
+      const int nk = g.kb[blk] >= 0 ? g.nch[blk] : 0;
+      // sums in units of 2^48 of the digits' least product weight (level 4);
+      // level 5 enters rounded to it
+      long long acc[32];
+#pragma unroll
+      for (int x = 0; x < 32; ++x) acc[x] = 0;
+      for (int c0 = 0; c0 < nk; c0 += kDgDrain, ++drain) {
+        ok = mbar_wait(&bar_accf, drain & 1u, g.wait_ns);
+        ok = __all_sync(0xffffffffu, ok && !s_abort);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * hc);
+#pragma unroll
+        for (int x = 0; x < 32; x += 8)
+          if (x < hc) {
+            float v[kDgS][8];
+            dg_ld8x6(ta + (uint32_t)x, (uint32_t)BN, v);
+#pragma unroll
+            for (int y = 0; y < 8; ++y) {
+              const int l4 = __float2int_rn(fmaf(v[5][y], 0.00390625f, v[4][y]));
+              long long s = acc[x + y] + l4;
+              s += (long long)__float2int_rn(v[3][y]) * 256;
+              s += (long long)__float2int_rn(v[2][y]) * 65536;
+              s += (long long)__float2int_rn(v[1][y]) * 16777216;
+              s += (long long)__float2int_rn(v[0][y]) << 32;
+              acc[x + y] = s;
+            }
+          }
+        tc_fence_before();
+        mbar_arrive(&bar_acce);
+      }
+      if (!ok) {
+        s_abort = 1;
+        break;
+      }
+      const int r = blk * kTcRows + q * 32 + lane;
+      if (r >= g.R) continue;
+      // value = acc * 2^(rowexp + colexp - 2090)
+      const int er = g.rowexp[r] - 1045;
+      const double sr = er < -1022 ? 0.0 : __longlong_as_double((long long)(er + 1023) << 52);
+      const int n0 = nt * BN + half * hc;
+      const int64_t o0 = (int64_t)r * N;
+#pragma unroll
+      for (int x = 0; x < 32; ++x) {
+        const int n = n0 + x;
+        if (x >= hc || n >= N) continue;
+        const int ce = g.colexp[n], ec = ce - 1045;
+        const double sc = ec < -1022 ? 0.0 : __longlong_as_double((long long)(ec + 1023) << 52);
+        double v = (double)acc[x] * sr * sc;
+        if (ce == 2047) v = dg_plain<MODE == 4>(g, r, n);
+        const int64_t o = o0 + n;
+        if (MODE == 0) {
+          g.out[o] = 2.0 * (v - g.P[o]);
+        } else if (MODE == 3) {
+          g.out[o] = v - g.P[o];
+        } else {
+          if (g.c2gam != 0.0) {
+            const double vi = g.V[o];
+            if (r < g.R - 1) v = fma(g.c2gam, vi - g.V[o + N], v);
+            if (r > 0) v = fma(-g.c2gam, g.V[o - N] - vi, v);
+          }
+          if (g.out) g.out[o] = v;
+          if (g.out2) g.out2[o] = v;
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (s_abort && threadIdx.x == 0) {
+    *g.err = 1.0;
+    for (int it = s_consumed; it < s_issued; ++it)
+      if (!mbar_wait(&bar_full[it % stages], (uint32_t)(it / stages) & 1u, g.wait_ns)) break;
+    mbar_wait(&bar_fin, 0, g.wait_ns);
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tc_dealloc(tmem, ncols);
+  }
+}
+
+}  // namespace pqdts
