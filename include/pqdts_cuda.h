@@ -85,8 +85,12 @@ int pqdts_cuda_kernel_launches(pqdts_ctx* ctx, int64_t* count);
  *              double-FP32 check) as one tensor-core product over all
  *              probes' columns wherever the CG's products run on the tensor
  *              cores; 0: FP32 CUDA-core tiles.
- *   "df_products" -1 (default, auto) / 1: the mixed path's gradient F^T.R
- *              and its objective checks (residual F.X - P) in double-FP32
+ *   "df_products" -1 (default, auto): the mixed path's gradient F^T.R
+ *              and its objective checks (residual F.X - P) by exact digits
+ *              on the tensor cores where those are in use ("tensor_cores")
+ *              and F is finite (48 bits of each row's and column's scale,
+ *              error ~sqrt(K) * 2^-47 of their product for K terms), else as
+ *              1: in double-FP32
  *              (pairs of FP32 numbers, ~sqrt(K) * 2^-48 relative to the
  *              sum of the K terms' magnitudes) on the CUDA cores; 0: native
  *              FP64.  Takes
@@ -123,7 +127,8 @@ int pqdts_cuda_set_option(pqdts_ctx* ctx, const char* name, int64_t value);
  * "sched.tc_splits" (K segments of their F^T product), "sched.tc_splits1"
  * (of their F.V product), "sched.tc_persistent" (kernel form),
  * "sched.df_fwd", "sched.df_trans" (double-FP32 residual / gradient
- * products in use), "sched.tc_screen" (line-search probe products on the
+ * products in use, or their digit forms), "sched.dg_fwd", "sched.dg_trans"
+ * (digit products in use), "sched.tc_screen" (line-search probe products on the
  * tensor cores), "graphs.captured" (graphs held). */
 int pqdts_cuda_get_option(pqdts_ctx* ctx, const char* name, int64_t* value);
 /* verbose = 1 prints the reference's stdout lines (iter, newton-pcg, line

@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <map>
 #include <memory>
@@ -33,6 +34,7 @@
 #include "kernels.cuh"
 #include "problem_host.h"
 #include "tc_band.cuh"
+#include "tc_digits.cuh"
 #include "batch_cg.cuh"
 
 namespace pqdts {
@@ -295,6 +297,17 @@ struct TcOperand {
   std::map<std::array<int, 3>, std::unique_ptr<TcSched>> scheds;  // keyed by (BN, splits, N)
 };
 
+// Band operand of the digit products: the digits of a TcOperand's row blocks
+// (same K windows), each row's exponent, the product's N tile width and tile
+// lists, and the B operand's map for that width.
+struct DgOperand {
+  DBuf<uint16_t> dig;
+  DBuf<int> rowexp;
+  CUtensorMap map_a, map_b;
+  TcSched sched;
+  int bn = 0, stages = 0;
+};
+
 // CG work vectors of one precision.
 template <typename T>
 struct CGBufs {
@@ -380,6 +393,13 @@ struct pqdts_ctx {
   int df_option = -1;
   int df_rows = 0;  // band rows per block of the double-FP32 products (0: chosen by size)
   bool df_fwd = false, df_trans = false;
+  // the same products by exact digits on the tensor cores (tc_digits.cuh):
+  // F's and F^T's digits, those of X and R (K-major) and their columns'
+  // exponents
+  bool dg_fwd = false, dg_trans = false;
+  pqdts::DgOperand dgF, dgFt;
+  pqdts::DBuf<uint16_t> dg_x, dg_r;
+  pqdts::DBuf<int> dg_colexp;
   bool exact = true;  // FP64: every reduction in the oracle's order
   pqdts::DBuf<int> ipart;
   pqdts::DBuf<long long> icount;
@@ -531,11 +551,26 @@ static void read_back(Ctx& c, const double* dev, int count) {
 // barrier wait ran out has set SC_TCERR.  The flag is cleared (the kernels
 // freed their tensor memory and stored nothing, the context stays usable)
 // and the call fails with PQDTS_E_CUDA.
-static void check_tc_error(Ctx& c) {
-  if (c.pin[SC_TCERR] == 0.0) return;
+static void throw_tc_error(Ctx& c) {
   CK(cudaMemsetAsync(c.sc.p + SC_TCERR, 0, sizeof(double), c.st));
   CK(cudaStreamSynchronize(c.st));
+  // what the product was to write is not there
+  c.R_ver = c.G_ver = c.Gf_ver = c.L_ver = -1;
   throw Err(PQDTS_E_CUDA, "tensor-core product: a barrier wait timed out");
+}
+
+static void check_tc_error(Ctx& c) {
+  if (c.pin[SC_TCERR] != 0.0) throw_tc_error(c);
+}
+
+// Waits for the stream; on a context whose gradient and objective products
+// run on the tensor cores, also checks that none of them gave up.
+static void check_products(Ctx& c) {
+  constexpr int kAt = 48;  // scalars' place in the pinned buffer, past every other read-back
+  if (c.dg_fwd)
+    CK(cudaMemcpyAsync(c.pin + kAt, c.sc.p + SC_TCERR, sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  CK(cudaStreamSynchronize(c.st));
+  if (c.dg_fwd && c.pin[kAt] != 0.0) throw_tc_error(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -573,6 +608,17 @@ static float2 split_df_host(double v) {
   return make_float2(h, (float)(v - (double)h));
 }
 
+// Whether the mixed path's tensor-core products are to be set up (the option
+// allows them and the device is a tcgen05 part).
+static bool tc_wanted(const Ctx& c) {
+  if (c.precision != PQDTS_MIXED || c.tc_option == 0) return false;
+  int major = 0;
+  CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, c.device));
+  if (major != 10 && c.tc_option == 1)
+    throw Err(PQDTS_E_ARG, "tensor-core products need a compute capability 10.x device");
+  return major == 10;
+}
+
 static void setup_device(Ctx& c) {
   HostProblem& h = c.h;
   const int64_t M = h.M, N = h.N, D = h.D, MN = M * N;
@@ -586,6 +632,7 @@ static void setup_device(Ctx& c) {
   c.tval.upload(h.tval.data(), h.tval.size(), c.st, &c.h2d);
   c.bdiag.upload(h.bdiag.data(), M, c.st, &c.h2d);
   c.P.upload(h.P.data(), h.P.size(), c.st, &c.h2d);
+  c.f_finite = std::all_of(h.fval.begin(), h.fval.end(), [](double v) { return std::isfinite(v); });
   c.t_contiguous = true;
   for (int64_t i = 0; i < M && c.t_contiguous; ++i) {
     const int64_t e0 = h.tptr[i], e1 = h.tptr[i + 1];
@@ -612,7 +659,11 @@ static void setup_device(Ctx& c) {
     c.df_fwd = c.df_option != 0;
     c.df_trans = c.df_fwd && c.t_contiguous;
     CK(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
-    if (c.df_fwd) {
+    // by digits on the tensor cores unless double-FP32 (df_products = 1) or
+    // CUDA cores (tensor_cores = 0) are asked for; a digit needs a finite F
+    c.dg_fwd = c.df_option < 0 && c.f_finite && tc_wanted(c);
+    c.dg_trans = c.dg_fwd && c.t_contiguous;
+    if (c.df_fwd && !c.dg_fwd) {
       std::vector<float2> fd(h.fval.size());
       for (size_t k = 0; k < fd.size(); ++k) fd[k] = split_df_host(h.fval[k]);
       c.fdf.upload(fd.data(), fd.size(), c.st, &c.h2d);
@@ -621,7 +672,7 @@ static void setup_device(Ctx& c) {
       c.fdf.release();
       c.xdf.release();
     }
-    if (c.df_trans) {
+    if (c.df_trans && !c.dg_trans) {
       std::vector<float2> td(h.tval.size());
       for (size_t k = 0; k < td.size(); ++k) td[k] = split_df_host(h.tval[k]);
       c.tdf.upload(td.data(), td.size(), c.st, &c.h2d);
@@ -639,11 +690,10 @@ static void setup_device(Ctx& c) {
     c.tdf.release();
     c.xdf.release();
     c.rdf.release();
-    c.df_fwd = c.df_trans = false;
+    c.df_fwd = c.df_trans = c.dg_fwd = c.dg_trans = false;
   }
   c.cg64.alloc(MN, M, D * N);
   c.sqd.alloc(M);
-  c.f_finite = std::all_of(h.fval.begin(), h.fval.end(), [](double v) { return std::isfinite(v); });
   c.xmask.alloc((size_t)kBatchLS * cdiv(N, 32) * cdiv(M, 32));
   c.rmask.alloc((size_t)N * cdiv(D, 32));
   if (c.t_contiguous && c.f_finite) {
@@ -867,11 +917,60 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
 }
 
 
-// Residual of X (FP64, M x N) in double-FP32: MODE 0 R = 2*(F.X - P),
-// MODE 3 R = F.X - P.
+// The mixed path's digit products read `rows` x N doubles of B as digits of
+// each column's scale: the columns' exponents, then the transposed digits.
+static void dg_split(Ctx& c, const double* B, int rows, int64_t ld, DBuf<uint16_t>& dig) {
+  const int N = (int)c.h.N;
+  CK(cudaMemsetAsync(c.dg_colexp.p, 0, N * sizeof(int), c.st));
+  // ~4 blocks per SM, at least 64 rows each
+  const int shares = std::max(1, std::min(cdiv(rows, 64), cdiv((int64_t)4 * c.num_sms, cdiv(N, 32))));
+  k_dg_colexp<<<dim3(cdiv(N, 32), shares), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p);
+  post_launch(c);
+  k_dg_split_t<<<dim3(cdiv(rows, 64), cdiv(N, 32)), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p, ld, dig.p);
+  post_launch(c);
+}
+
+// One digit product: op's rows (`rows` of F or F^T) times the digits in
+// place, B their FP64 values; see k_dg_band_product for the modes.
+template <int MODE>
+static void dg_product(Ctx& c, DgOperand& op, TcOperand& win, int rows, const double* B, double* out, double* out2,
+                       const double* V, double c2gam) {
+  DgArgs g;
+  g.kb = win.kb.p;
+  g.nch = win.nch.p;
+  g.rowexp = op.rowexp.p;
+  g.colexp = c.dg_colexp.p;
+  g.sched_off = op.sched.off.p;
+  g.sched_tile = op.sched.tile.p;
+  g.R = rows;
+  g.N = (int)c.h.N;
+  g.BN = op.bn;
+  g.stages = op.stages;
+  g.P = c.P.p;
+  g.V = V;
+  g.c2gam = c2gam;
+  g.out = out;
+  g.out2 = out2;
+  g.f = bands_of(c);
+  g.val = MODE == 4 ? c.tval.p : c.fval.p;
+  g.B = B;
+  g.err = c.sc.p + SC_TCERR;
+  g.wait_ns = c.tc_wait_ns;
+  k_dg_band_product<MODE><<<op.sched.grid, kDgThreads, kDgRing + 1024, c.st>>>(op.map_a, op.map_b, g);
+  post_launch(c);
+}
+
+// Residual of X (FP64, M x N) to FP64 accuracy without the FP64 pipe: MODE 0
+// R = 2*(F.X - P), MODE 3 R = F.X - P.  By digits on the tensor cores where
+// those are in use, else in double-FP32.
 template <int MODE>
 static void fwd_df(Ctx& c, const double* X, double* R) {
   const int64_t MN = c.h.M * c.h.N;
+  if (c.dg_fwd) {
+    dg_split(c, X, (int)c.h.M, c.tc_mp, c.dg_x);
+    dg_product<MODE>(c, c.dgF, c.tcF, (int)c.h.D, X, R, nullptr, nullptr, 0.0);
+    return;
+  }
   require(c.xdf.p, "xdf");
   k_split_df<<<elem_grid(MN), 256, 0, c.st>>>(X, MN, 1.0, c.xdf.p);
   post_launch(c);
@@ -903,7 +1002,7 @@ static void objective_stack(Ctx& c, const double* Xs, int B) {
 
 static void fetch_objectives(Ctx& c, int B, double* L) {
   CK(cudaMemcpyAsync(c.pin, c.lsout.p, 4 * kBatchLS * sizeof(double), cudaMemcpyDeviceToHost, c.st));
-  CK(cudaStreamSynchronize(c.st));
+  check_products(c);
   for (int b = 0; b < B; ++b) L[b] = (c.h.gam != 0 && !c.exact) ? c.pin[b] + c.pin[kBatchLS + b] : c.pin[b];
 }
 
@@ -1057,22 +1156,27 @@ static void op_dL(Ctx& c) {
       post_launch(c);
     }
   } else if (c.df_trans) {
-    // mixed path, double-FP32: full-space gradient into Gf (and G), then
-    // the reduced one from it
+    // mixed path, digits or double-FP32: full-space gradient into Gf (and
+    // G), then the reduced one from it
     ensure_R(c);
     const int D = (int)c.h.D;
-    k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p);
-    post_launch(c);
     double* g = c.fullspace ? c.G.p : nullptr;
     const double c2g = 2.0 * c.h.gam;
-    const int rb = df_rows_per_block(M, N, c.df_rows, c.num_sms);
-    const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
-    const dim3 grid(cdiv(M, rb), cdiv(N, threads));
-    DevBands bd = bands_of(c);
-    if (rb == 8) k_trans_df<8><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
-    else if (rb == 4) k_trans_df<4><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
-    else k_trans_df<2><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
-    post_launch(c);
+    if (c.dg_trans) {
+      dg_split(c, c.R.p, D, c.tc_dp, c.dg_r);
+      dg_product<4>(c, c.dgFt, c.tcFt, M, c.R.p, c.Gf.p, g, c.X.p, c2g);
+    } else {
+      k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p);
+      post_launch(c);
+      const int rb = df_rows_per_block(M, N, c.df_rows, c.num_sms);
+      const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
+      const dim3 grid(cdiv(M, rb), cdiv(N, threads));
+      DevBands bd = bands_of(c);
+      if (rb == 8) k_trans_df<8><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
+      else if (rb == 4) k_trans_df<4><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
+      else k_trans_df<2><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
+      post_launch(c);
+    }
     if (!c.fullspace) {
       k_reduced_from_full<<<M, std::min(256, std::max(32, cdiv(N, 32) * 32)), 0, c.st>>>(c.Gf.p, c.maxr.p, N, c.G.p);
       post_launch(c);
@@ -1260,13 +1364,7 @@ static void tc_configure(Ctx& c, int bn) {
 // option allows and the device is a tcgen05 part).
 static void setup_tc(Ctx& c) {
   c.tc_ready = false;
-  if (c.precision != PQDTS_MIXED || c.tc_option == 0) return;
-  int major = 0;
-  CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, c.device));
-  if (major != 10) {
-    if (c.tc_option == 1) throw Err(PQDTS_E_ARG, "tensor-core products need a compute capability 10.x device");
-    return;
-  }
+  if (!tc_wanted(c)) return;
   const HostProblem& h = c.h;
   const int64_t M = h.M, N = h.N, D = h.D;
   const int bn = tc_tile_n(N, 1);
@@ -1283,6 +1381,99 @@ static void setup_tc(Ctx& c) {
   CK(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
   tc_configure(c, bn);
   c.tc_ready = true;
+}
+
+// 3-D bf16 map of an operand's digits: inner x rows x kDgS, box kTcK x
+// box_rows x kDgS, swizzled to the stage's row width, zero fill outside.
+static void make_map_digits(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint64_t row_elems,
+                            uint32_t box_rows) {
+  const cuuint64_t dims[3] = {inner, rows, (cuuint64_t)kDgS};
+  const cuuint64_t strides[2] = {row_elems * 2, rows * row_elems * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)kTcK, box_rows, (cuuint32_t)kDgS};
+  const cuuint32_t es[3] = {1, 1, 1};
+  static_assert(kTcRowBytes == 64, "the swizzle below");
+  const CUresult r = encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
+                                    es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw Err(PQDTS_E_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+}
+
+// N tile width of a digit product over A's row blocks: the one of 64, 48,
+// 32, 16 (their six levels fit tensor memory) with the least estimated time,
+// waves of tiles x the cycles of a K chunk -- the larger of the MMAs'
+// (21 digit pairs x BN / 4 cycles a chunk) and shared memory's (128 bytes a
+// cycle: 4 KB of A per instruction, BN x 64 bytes of B per pair, twice a
+// chunk) -- so narrow tiles are taken only to fill the SMs.
+static int dg_tile_n(const Ctx& c, const TcOperand& A) {
+  const int N = (int)c.h.N;
+  int best = 16;
+  double least = 0.0;
+  for (int bn : {64, 48, 32, 16}) {
+    int instr = 0;
+    for (int p = 0; p < kDgS; ++p) instr += cdiv((kDgS - p) * bn, 256);
+    const int pairs = kDgS * (kDgS + 1) / 2;
+    const double cyc = std::max(pairs * bn, 64 * instr + pairs * bn / 2);
+    const double t = cyc * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
+    if (least == 0.0 || t < least) {
+      least = t;
+      best = bn;
+    }
+  }
+  return best;
+}
+
+// Digits of F (or F^T, trans) over win's row blocks and K windows, the tile
+// lists and the maps; dig_b: the other operand's digits, K x N, ld apart.
+static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf<uint16_t>& dig_b, int64_t K,
+                         int64_t ld) {
+  const int N = (int)c.h.N, rows = win.blocks * kTcRows;
+  op.dig.alloc((size_t)kDgS * rows * win.kmax);
+  op.rowexp.alloc(rows);
+  dig_b.alloc((size_t)kDgS * N * ld);
+  if (trans)
+    k_dg_band<true><<<rows, 256, 0, c.st>>>(bands_of(c), c.tval.p, win.kb.p, rows, win.kmax, op.dig.p, op.rowexp.p);
+  else
+    k_dg_band<false><<<rows, 256, 0, c.st>>>(bands_of(c), c.fval.p, win.kb.p, rows, win.kmax, op.dig.p, op.rowexp.p);
+  post_launch(c);
+  op.bn = dg_tile_n(c, win);
+  const uint32_t stage = kDgS * (kTcRows + (uint32_t)op.bn) * kTcRowBytes;
+  op.stages = std::min<int>(kDgMaxStages, (int)(kDgRing / stage));
+  make_map_digits(&op.map_a, op.dig.p, win.kmax, rows, win.kmax, kTcRows);
+  make_map_digits(&op.map_b, dig_b.p, K, N, ld, (uint32_t)op.bn);
+  // tiles from the last row block down (the widest K windows of a Poisson F
+  // first), each to the CTA with the least work so far: the CTAs stay within
+  // a few row blocks of one another, so A's digits are read from HBM once
+  const int ntn = cdiv(N, op.bn), T = ntn * win.blocks, grid = std::min(T, c.num_sms);
+  std::vector<std::vector<int32_t>> lists(grid);
+  std::vector<std::pair<int64_t, int>> load(grid);  // heap: (work, CTA), least first
+  for (int g = 0; g < grid; ++g) load[g] = {0, g};
+  const auto more = std::greater<std::pair<int64_t, int>>();
+  for (int t = T - 1; t >= 0; --t) {
+    std::pop_heap(load.begin(), load.end(), more);
+    auto& l = load.back();
+    l.first += win.h_nch[t / ntn] + 4;
+    lists[l.second].push_back(t);
+    std::push_heap(load.begin(), load.end(), more);
+  }
+  std::vector<int32_t> off(grid + 1, 0), tiles;
+  for (int g = 0; g < grid; ++g) {
+    tiles.insert(tiles.end(), lists[g].begin(), lists[g].end());
+    off[g + 1] = (int32_t)tiles.size();
+  }
+  op.sched.grid = grid;
+  op.sched.off.upload(off.data(), off.size(), c.st, &c.h2d);
+  op.sched.tile.upload(tiles.data(), tiles.size(), c.st, &c.h2d);
+  CK(cudaStreamSynchronize(c.st));  // the host vectors go out of scope
+}
+
+static void setup_dg(Ctx& c) {
+  if (!c.dg_fwd) return;
+  c.dg_colexp.alloc(c.h.N);
+  CK(cudaFuncSetAttribute(k_dg_band_product<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
+  CK(cudaFuncSetAttribute(k_dg_band_product<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
+  CK(cudaFuncSetAttribute(k_dg_band_product<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
+  setup_digits(c, c.dgF, c.tcF, false, c.dg_x, c.h.M, c.tc_mp);
+  if (c.dg_trans) setup_digits(c, c.dgFt, c.tcFt, true, c.dg_r, c.h.D, c.tc_dp);
 }
 
 // Tile lists of the persistent kernel for A's row blocks at N tile width bn
@@ -2061,7 +2252,8 @@ static double op_conv(Ctx& c, bool tprint, bool with_extra = false) {
   } else {
     reduce_to(c, c.part.p, M, c.sc.p + SC_TMP);
   }
-  read_back(c, c.sc.p + SC_TMP, with_extra ? 2 : 1);
+  CK(cudaMemcpyAsync(c.pin, c.sc.p + SC_TMP, (with_extra ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  check_products(c);
   const double conv = std::sqrt(c.pin[0] / ((double)N * (double)M));
   if (tprint && c.verbose) {
     std::vector<double> hl(M), hg((size_t)M * N);
@@ -2789,6 +2981,7 @@ static void tune_schedule(Ctx& c, Schedule& s) {
 static void choose_schedule(Ctx& c) {
   const HostProblem& h = c.h;
   setup_tc(c);
+  setup_dg(c);
   Schedule s = heuristic_schedule(h);
   if (c.tc_ready) {
     s.tc = 1;
@@ -3128,6 +3321,7 @@ int pqdts_cuda_dL(pqdts_ctx* c, double* G) {
     pqdts::need_problem(*c);
     pqdts::op_dL(*c);
     pqdts::download_colmajor(*c, c->G.p, G);
+    pqdts::check_products(*c);
   });
 }
 
@@ -3529,6 +3723,8 @@ int pqdts_cuda_get_option(pqdts_ctx* c, const char* name, int64_t* value) {
     else if (n == "internal_f") *value = c->internal_f_option;
     else if (n == "sched.df_fwd") *value = c->df_fwd;
     else if (n == "sched.df_trans") *value = c->df_trans;
+    else if (n == "sched.dg_fwd") *value = c->dg_fwd;
+    else if (n == "sched.dg_trans") *value = c->dg_trans;
     else if (n == "sched.tc_screen") *value = (s.tc && c->tc_ready && c->tc_screen_option != 0) ? 1 : 0;
     else if (n == "graphs.captured") *value = (int64_t)c->graphs.size();
     else throw pqdts::Err(PQDTS_E_ARG, "unknown option " + n);
