@@ -340,6 +340,8 @@ struct pqdts_ctx {
   pqdts::DBuf<int32_t> flo, fw, tidx;
   pqdts::DBuf<int64_t> foff, tptr;
   pqdts::DBuf<double> fval, tval, bdiag, P;
+  pqdts::DBuf<double> tbval;  // F^T's band values where a column's d have gaps
+  const double* tband_values() const { return t_contiguous ? tval.p : tbval.p; }
   pqdts::DBuf<float> fval32, tval32, tbval32, rsq32;
   pqdts::DBuf<double> sqd;  // sqrt(bdfac * Bdiag) per row, FP64 CG step
   bool t_contiguous = false;  // every column of F supported on a contiguous range of d
@@ -602,12 +604,6 @@ static void launch_fwd_df(Ctx& c, double* R, const uint32_t* xmask) {
 }
 
 
-// (hi, lo) FP32 pair of an FP64 value, as k_split_df forms it on the device.
-static float2 split_df_host(double v) {
-  const float h = (float)v;
-  return make_float2(h, (float)(v - (double)h));
-}
-
 // Whether the mixed path's tensor-core products are to be set up (the option
 // allows them and the device is a tcgen05 part).
 static bool tc_wanted(const Ctx& c) {
@@ -619,36 +615,67 @@ static bool tc_wanted(const Ctx& c) {
   return major == 10;
 }
 
-static void setup_device(Ctx& c) {
+// The problem's arrays on the device (maxr_state: the seeded stream before
+// the first maxr's draws) and the work buffers.
+static void setup_device(Ctx& c, uint64_t maxr_state) {
   HostProblem& h = c.h;
   const int64_t M = h.M, N = h.N, D = h.D, MN = M * N;
   c.drop_graphs();  // their kernels hold the buffers about to be replaced
+  const int64_t nnz = h.nnz();
   c.flo.upload(h.flo.data(), D, c.st, &c.h2d);
   c.fw.upload(h.fw.data(), D, c.st, &c.h2d);
   c.foff.upload(h.foff.data(), D, c.st, &c.h2d);
-  c.fval.upload(h.fval.data(), h.fval.size(), c.st, &c.h2d);
+  c.fval.upload(h.values(), nnz, c.st, &c.h2d);
   c.tptr.upload(h.tptr.data(), h.tptr.size(), c.st, &c.h2d);
-  c.tidx.upload(h.tidx.data(), h.tidx.size(), c.st, &c.h2d);
-  c.tval.upload(h.tval.data(), h.tval.size(), c.st, &c.h2d);
-  c.bdiag.upload(h.bdiag.data(), M, c.st, &c.h2d);
-  c.P.upload(h.P.data(), h.P.size(), c.st, &c.h2d);
-  c.f_finite = std::all_of(h.fval.begin(), h.fval.end(), [](double v) { return std::isfinite(v); });
-  c.t_contiguous = true;
-  for (int64_t i = 0; i < M && c.t_contiguous; ++i) {
-    const int64_t e0 = h.tptr[i], e1 = h.tptr[i + 1];
-    if (e1 > e0 && h.tidx[e1 - 1] - h.tidx[e0] + 1 != e1 - e0) c.t_contiguous = false;
+  c.tlo.upload(h.tlo.data(), M, c.st, &c.h2d);
+  c.tw.upload(h.tw.data(), M, c.st, &c.h2d);
+  c.toff.upload(h.toff.data(), M, c.st, &c.h2d);
+  c.P.upload(h.P_data(), (size_t)D * N, c.st, &c.h2d);
+  c.tval.alloc(nnz);
+  c.tidx.alloc(nnz);
+  c.bdiag.alloc(M);
+  c.t_contiguous = h.t_contiguous;
+  // the transposed values, on the device unless a column's d have gaps (the
+  // scatter is then in the host's order)
+  if (h.t_contiguous) {
+    k_transpose_bands<<<cdiv(M, 8), 256, 0, c.st>>>(bands_of(c), c.fval.p, c.tlo.p, c.tval.p, c.tidx.p);
+    post_launch(c);
+  } else {
+    transpose_with_gaps(h, c.precision == PQDTS_MIXED);
+    c.tidx.upload(h.tidx.data(), h.tidx.size(), c.st, &c.h2d);
+    c.tval.upload(h.tval.data(), h.tval.size(), c.st, &c.h2d);
   }
+  k_bdiag<<<cdiv(M, 32), 32, 0, c.st>>>(bands_of(c), c.tval.p, h.gam, c.bdiag.p);
+  post_launch(c);
+  c.maxr.alloc(M);
+  k_initial_maxr<<<cdiv(M, 32), 32, 0, c.st>>>(maxr_state, (int)M, (int)N, c.maxr.p);
+  post_launch(c);
+  c.ipart.alloc(kElemGrid);
+  CK(cudaMemsetAsync(c.ipart.p, 0, sizeof(int), c.st));
+  k_any_not_finite<<<elem_grid(nnz), 256, 0, c.st>>>(c.fval.p, nnz, c.ipart.p);
+  post_launch(c);
+  int not_finite = 0;
+  h.bdiag.resize(M);
+  c.h_maxr.resize(M);
+  CK(cudaMemcpyAsync(h.bdiag.data(), c.bdiag.p, M * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  CK(cudaMemcpyAsync(c.h_maxr.data(), c.maxr.p, M * sizeof(int32_t), cudaMemcpyDeviceToHost, c.st));
+  CK(cudaMemcpyAsync(&not_finite, c.ipart.p, sizeof(int), cudaMemcpyDeviceToHost, c.st));
+  CK(cudaStreamSynchronize(c.st));
+  c.f_finite = not_finite == 0;
   if (c.precision == PQDTS_MIXED) {
-    std::vector<float> f32(h.fval.begin(), h.fval.end());
-    c.fval32.upload(f32.data(), f32.size(), c.st, &c.h2d);
-    std::vector<float> t32(h.tval.begin(), h.tval.end());
-    c.tval32.upload(t32.data(), t32.size(), c.st, &c.h2d);
-    transposed_bands(h);
-    c.tlo.upload(h.tlo.data(), h.tlo.size(), c.st, &c.h2d);
-    c.tw.upload(h.tw.data(), h.tw.size(), c.st, &c.h2d);
-    c.toff.upload(h.toff.data(), h.toff.size(), c.st, &c.h2d);
-    std::vector<float> tb32(h.tbval.begin(), h.tbval.end());
-    c.tbval32.upload(tb32.data(), tb32.size(), c.st, &c.h2d);
+    c.fval32.alloc(nnz);
+    c.tval32.alloc(nnz);
+    k_to_float<<<elem_grid(nnz), 256, 0, c.st>>>(c.fval.p, nnz, c.fval32.p);
+    post_launch(c);
+    k_to_float<<<elem_grid(nnz), 256, 0, c.st>>>(c.tval.p, nnz, c.tval32.p);
+    post_launch(c);
+    // F^T's band form: the transposed values as they are, or with its gaps
+    if (!h.t_contiguous) c.tbval.upload(h.tbval.data(), h.tbval.size(), c.st, &c.h2d);
+    else c.tbval.release();
+    const int64_t ntb = h.t_contiguous ? nnz : (int64_t)h.tbval.size();
+    c.tbval32.alloc(ntb);
+    k_to_float<<<elem_grid(ntb), 256, 0, c.st>>>(c.tband_values(), ntb, c.tbval32.p);
+    post_launch(c);
     c.rsq32.alloc(M);
     c.cg32.alloc(MN, M, D * N);
     c.x0c.alloc(MN);
@@ -664,25 +691,25 @@ static void setup_device(Ctx& c) {
     c.dg_fwd = c.df_option < 0 && c.f_finite && tc_wanted(c);
     c.dg_trans = c.dg_fwd && c.t_contiguous;
     if (c.df_fwd && !c.dg_fwd) {
-      std::vector<float2> fd(h.fval.size());
-      for (size_t k = 0; k < fd.size(); ++k) fd[k] = split_df_host(h.fval[k]);
-      c.fdf.upload(fd.data(), fd.size(), c.st, &c.h2d);
+      c.fdf.alloc(nnz);
+      k_split_df<<<elem_grid(nnz), 256, 0, c.st>>>(c.fval.p, nnz, 1.0, c.fdf.p);
+      post_launch(c);
       c.xdf.alloc(MN);
     } else {
       c.fdf.release();
       c.xdf.release();
     }
     if (c.df_trans && !c.dg_trans) {
-      std::vector<float2> td(h.tval.size());
-      for (size_t k = 0; k < td.size(); ++k) td[k] = split_df_host(h.tval[k]);
-      c.tdf.upload(td.data(), td.size(), c.st, &c.h2d);
+      c.tdf.alloc(nnz);
+      k_split_df<<<elem_grid(nnz), 256, 0, c.st>>>(c.tval.p, nnz, 1.0, c.tdf.p);
+      post_launch(c);
       c.rdf.alloc(D * N);
     } else {
       c.tdf.release();
       c.rdf.release();
     }
-    CK(cudaStreamSynchronize(c.st));  // host staging vectors go out of scope
   } else {
+    c.tbval.release();
     c.fval32.release();
     c.tval32.release();
     c.tbval32.release();
@@ -704,10 +731,9 @@ static void setup_device(Ctx& c) {
     for (int64_t b = 0; b < nb; ++b) {
       int32_t l = INT32_MAX, u = 0;
       for (int64_t i = b * 32; i < std::min(M, b * 32 + 32); ++i) {
-        const int64_t e0 = h.tptr[i], e1 = h.tptr[i + 1];
-        if (e1 > e0) {
-          l = std::min(l, h.tidx[e0]);
-          u = std::max(u, h.tidx[e1 - 1] + 1);
+        if (h.tlo[i] >= 0) {
+          l = std::min(l, h.tlo[i]);
+          u = std::max(u, h.tlo[i] + h.tw[i]);
         }
       }
       if (l >= u) l = u = 0;
@@ -792,12 +818,10 @@ static void setup_device(Ctx& c) {
   c.R.alloc(D * N);
   c.sn64.alloc(MN);
   c.ik.alloc(MN);
-  c.maxr.alloc(M);
   const int64_t fwd_parts = (int64_t)cdiv(N, kBX) * cdiv(D, kBY) * kBatchLS;
   const int64_t np = std::max<int64_t>({fwd_parts, M, (int64_t)kElemGrid * kBatchLS, 1024});
   c.part.alloc(np);
   c.part2.alloc(np);
-  c.ipart.alloc(kElemGrid);
   c.icount.alloc(1);
   c.sc.alloc(SC_NSC);
   CK(cudaMemsetAsync(c.sc.p, 0, SC_NSC * sizeof(double), c.st));
@@ -809,8 +833,6 @@ static void setup_device(Ctx& c) {
   post_launch(c);
   c.R_ver = c.G_ver = c.L_ver = c.rebuilt_ver = c.Gf_ver = -1;
   touch_x(c);
-  CK(cudaMemcpyAsync(c.maxr.p, c.h_maxr.data(), M * 4, cudaMemcpyHostToDevice, c.st));
-  c.h2d += M * 4;
   CK(cudaStreamSynchronize(c.st));
   c.fullspace = true;
   c.have_problem = true;
@@ -1283,11 +1305,12 @@ static void make_map_bf16(CUtensorMap* m, const void* base, uint64_t inner, uint
   if (r != CUDA_SUCCESS) throw Err(PQDTS_E_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
 }
 
-// Band rows (lo / w / off / val over R rows, FP64) as a TcOperand: values
-// split into bf16 hi + lo (hi = bf16(v), lo = bf16(v - hi)).
+// Band rows (lo / w over R rows; their offsets and FP64 values on the device)
+// as a TcOperand: values split into bf16 hi + lo (hi = bf16(v), lo = bf16(v -
+// hi)).
 static void build_tc_operand(Ctx& c, const std::vector<int32_t>& lo, const std::vector<int32_t>& w,
-                             const std::vector<int64_t>& off, const std::vector<double>& val, int64_t R,
-                             TcOperand& op) {
+                             const int32_t* d_lo, const int32_t* d_w, const int64_t* d_off, const double* d_val,
+                             int64_t R, TcOperand& op) {
   const int blocks = cdiv(R, kTcRows);
   std::vector<int32_t> kb(blocks, -1), nch(blocks, 0);
   int kmax = kTcK;
@@ -1305,28 +1328,20 @@ static void build_tc_operand(Ctx& c, const std::vector<int32_t>& lo, const std::
     kmax = std::max(kmax, nch[b] * kTcK);
   }
   const size_t total = (size_t)blocks * kTcRows * kmax;
-  std::vector<__nv_bfloat16> hv(total, __float2bfloat16(0.0f)), lv(total, __float2bfloat16(0.0f));
-  for (int64_t r = 0; r < R; ++r) {
-    const int b = (int)(r / kTcRows);
-    for (int k = 0; k < w[r]; ++k) {
-      const size_t x = (size_t)r * kmax + (size_t)(lo[r] + k - kb[b]);
-      const double v = val[off[r] + k];
-      const __nv_bfloat16 h = __double2bfloat16(v);
-      hv[x] = h;
-      lv[x] = __double2bfloat16(v - (double)__bfloat162float(h));
-    }
-  }
-  op.hi.upload(hv.data(), total, c.st, &c.h2d);
-  op.lo.upload(lv.data(), total, c.st, &c.h2d);
+  op.hi.alloc(total);
+  op.lo.alloc(total);
   op.kb.upload(kb.data(), blocks, c.st, &c.h2d);
   op.nch.upload(nch.data(), blocks, c.st, &c.h2d);
+  k_tc_split_band<<<blocks * kTcRows, 256, 0, c.st>>>(d_lo, d_w, d_off, d_val, op.kb.p, (int)R, kmax, op.hi.p,
+                                                      op.lo.p);
+  post_launch(c);
   op.h_nch = nch;
   op.scheds.clear();
   op.blocks = blocks;
   op.kmax = kmax;
   make_map_bf16(&op.map_hi, op.hi.p, kmax, (uint64_t)blocks * kTcRows, (uint64_t)kmax * 2, kTcK, kTcRows);
   make_map_bf16(&op.map_lo, op.lo.p, kmax, (uint64_t)blocks * kTcRows, (uint64_t)kmax * 2, kTcK, kTcRows);
-  CK(cudaStreamSynchronize(c.st));  // the host staging vectors go out of scope
+  CK(cudaStreamSynchronize(c.st));  // the host vectors go out of scope
 }
 
 // Tile width over N: N split in mult * ceil(N/256) equal tiles, rounded up
@@ -1368,8 +1383,8 @@ static void setup_tc(Ctx& c) {
   const HostProblem& h = c.h;
   const int64_t M = h.M, N = h.N, D = h.D;
   const int bn = tc_tile_n(N, 1);
-  build_tc_operand(c, h.flo, h.fw, h.foff, h.fval, D, c.tcF);
-  build_tc_operand(c, h.tlo, h.tw, h.toff, h.tbval, M, c.tcFt);
+  build_tc_operand(c, h.flo, h.fw, c.flo.p, c.fw.p, c.foff.p, c.fval.p, D, c.tcF);
+  build_tc_operand(c, h.tlo, h.tw, c.tlo.p, c.tw.p, c.toff.p, c.tband_values(), M, c.tcFt);
   c.tc_mp = (M + 7) / 8 * 8;
   c.tc_dp = (D + 7) / 8 * 8;
   c.vt_hi.alloc((size_t)N * c.tc_mp);
@@ -3054,6 +3069,7 @@ static void bands_internal_device(Ctx& c, HostProblem& h) {
   CK(cudaMemcpyAsync(h.fw.data(), w.p, (size_t)D * 4, cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
   finish_offsets(h);
+  h.fval.assign(h.total, 0.0);
   if (h.fval.empty()) return;
   off.upload(h.foff.data(), D, c.st, nullptr);
   val.alloc(h.fval.size());
@@ -3068,11 +3084,23 @@ static void init_problem(Ctx& c, HostProblem&& h, int precision, SeededStream& r
   if (precision != PQDTS_FP64 && precision != PQDTS_MIXED) throw Err(PQDTS_E_ARG, "precision must be 0 or 1");
   c.have_problem = false;
   c.h = std::move(h);
-  finish_problem(c.h);
-  c.h_maxr = initial_maxr(c.h.M, c.h.N, rng);
   c.precision = precision;
-  setup_device(c);
-  choose_schedule(c);
+  try {
+    column_ranges(c.h);
+    setup_device(c, rng.s);
+    choose_schedule(c);
+  } catch (...) {
+    cudaStreamSynchronize(c.st);  // no copy from the caller's arrays outlives the call
+    c.h.vals = c.h.Pin = nullptr;
+    throw;
+  }
+  // everything is on the device: the host's copies (and the caller's) go
+  c.h.vals = c.h.Pin = nullptr;
+  std::vector<double>().swap(c.h.fval);
+  std::vector<double>().swap(c.h.P);
+  std::vector<double>().swap(c.h.tval);
+  std::vector<double>().swap(c.h.tbval);
+  std::vector<int32_t>().swap(c.h.tidx);
 }
 
 static void check_sizes(int64_t M, int64_t N, int64_t D) {
@@ -3202,7 +3230,7 @@ int pqdts_cuda_set_problem(pqdts_ctx* c, int64_t M, int64_t N, int64_t D, const 
       if (lo[d] >= 0) tot += hi[d] - lo[d] + 1;
     if (tot > 0 && !vals) throw Err(PQDTS_E_ARG, "null band values");
     pqdts::bands_from_bands(h, lo, hi, vals);
-    h.P.assign(P, P + (size_t)D * N);
+    h.Pin = P;
     pqdts::SeededStream rng;
     pqdts::init_problem(*c, std::move(h), precision, rng);
   });

@@ -1,6 +1,9 @@
-// Host-side construction of a problem: F bands, P, the transposed CSR and
-// the Hessian diagonal.  All of it is set-up work done once per problem, in
-// O(nnz) (the reference's band build is O(D*nnz), pqdts.f90:1328-1364).
+// Host-side construction of a problem: F's bands and P from the caller's
+// formats, and the index arrays of F^T, O(D + M) where every column of F is
+// supported on a contiguous range of d.  The value arrays derived from F
+// (transposed, FP32, bf16, digits), the Hessian diagonal and the first maxr
+// are then built on the device.  (The reference's band build is O(D*nnz),
+// pqdts.f90:1328-1364.)
 #pragma once
 
 #include <algorithm>
@@ -18,18 +21,25 @@ struct HostProblem {
   double gam = 0.0;
   std::vector<int32_t> flo, fw;  // band start (-1 = empty row) and width
   std::vector<int64_t> foff;
-  std::vector<double> fval;
-  std::vector<double> P;         // (D, N) row-major
+  std::vector<double> fval;      // band values and P (D, N) row-major, where
+  std::vector<double> P;         // they were built here ...
+  const double* vals = nullptr;  // ... or the caller's, for the set-up call only
+  const double* Pin = nullptr;
   std::vector<int64_t> tptr;     // transposed CSR over columns i of F
-  std::vector<int32_t> tidx;
+  bool t_contiguous = true;      // every column i is in the bands of a contiguous range of d
+  std::vector<int32_t> tidx;     // (empty when t_contiguous)
   std::vector<double> tval;
   std::vector<double> bdiag;     // full-space Hessian diagonal, one value per row i
   // F^T as dense bands over d (zero filled where column i is not in row d's
-  // band): the mixed-precision tiled product's operand.
+  // band): first d (-1: none), width, offset; the values are the transposed
+  // CSR's when t_contiguous
   std::vector<int32_t> tlo, tw;
   std::vector<int64_t> toff;
   std::vector<double> tbval;
-  int64_t nnz() const { return (int64_t)fval.size(); }
+  int64_t total = 0;             // band entries
+  int64_t nnz() const { return total; }
+  const double* values() const { return vals ? vals : fval.data(); }
+  const double* P_data() const { return Pin ? Pin : P.data(); }
 };
 
 // splitmix64 uniform [0,1) stream seeded with 23764 (the reference's seed,
@@ -54,7 +64,7 @@ inline void finish_offsets(HostProblem& h) {
     h.foff[d] = tot;
     tot += h.fw[d];
   }
-  h.fval.assign(tot, 0.0);
+  h.total = tot;
 }
 
 // Bands from COO: [min col, max col] per row, zero filled, duplicates
@@ -74,6 +84,7 @@ inline void bands_from_coo(HostProblem& h, int64_t nnz, const int32_t* row, cons
   for (int64_t d = 0; d < h.D; ++d)
     if (h.flo[d] >= 0) h.fw[d] = hi[d] - h.flo[d] + 1;
   finish_offsets(h);
+  h.fval.assign(h.total, 0.0);
   for (int64_t k = 0; k < nnz; ++k) h.fval[h.foff[row[k]] + col[k] - h.flo[row[k]]] = val[k];
 }
 
@@ -87,7 +98,7 @@ inline void bands_from_bands(HostProblem& h, const int64_t* lo, const int64_t* h
     h.fw[d] = (int32_t)(hi[d] - lo[d] + 1);
   }
   finish_offsets(h);
-  std::copy(vals, vals + h.fval.size(), h.fval.begin());
+  h.vals = vals;
 }
 
 // fprob (pqdts.f90:188-206): Poisson pmf for mean < 50, Gaussian otherwise.
@@ -129,6 +140,7 @@ inline void bands_internal(HostProblem& h) {
     }
   }
   finish_offsets(h);
+  h.fval.assign(h.total, 0.0);
   for (int64_t d = 0; d < h.D; ++d)
     for (int64_t k = 0; k < h.fw[d]; ++k) h.fval[h.foff[d] + k] = fprob((double)(h.flo[d] + k), (double)mean_of[d]);
 }
@@ -147,10 +159,11 @@ inline void P_from_coo(HostProblem& h, int64_t nnz, const int32_t* row, const in
   }
 }
 
-// Transposed CSR (ascending d per column i) and the full-space Hessian
-// diagonal in the reference's order: 2*f^2 summed over ascending d, then
-// +2*gamma on rows 1..M-1, then +2*gamma on rows 2..M (pqdts.f90:214-234).
-inline void finish_problem(HostProblem& h) {
+// The columns' row ranges: tptr (entries per column), tlo / tw (first d and
+// the span to the last one) and whether every column's d are contiguous.
+// Each column takes its first d from the first band that covers it, found by
+// skipping covered columns, and its last one from the last: O(D + M).
+inline void column_ranges(HostProblem& h) {
   if ((int64_t)h.M * h.N >= (int64_t)1 << 31) throw std::invalid_argument("M*N must be below 2^31");
   std::vector<int64_t> cnt(h.M + 1, 0);
   for (int64_t d = 0; d < h.D; ++d)
@@ -164,6 +177,45 @@ inline void finish_problem(HostProblem& h) {
     run += cnt[i];
     h.tptr[i + 1] = h.tptr[i] + run;
   }
+  std::vector<int32_t> next(h.M + 1);
+  auto cover = [&](int64_t d, std::vector<int32_t>& out) {  // columns of band d not yet covered
+    if (h.fw[d] <= 0) return;
+    const int32_t hi = h.flo[d] + h.fw[d];
+    auto find = [&](int32_t i) {
+      while (next[i] != i) i = next[i] = next[next[i]];
+      return i;
+    };
+    for (int32_t i = find(h.flo[d]); i < hi; i = find(i)) {
+      out[i] = (int32_t)d;
+      next[i] = i + 1;
+    }
+  };
+  auto reset = [&] {
+    for (int64_t i = 0; i <= h.M; ++i) next[i] = (int32_t)i;
+  };
+  h.tlo.assign(h.M, -1);
+  std::vector<int32_t> last(h.M, -1);
+  reset();
+  for (int64_t d = 0; d < h.D; ++d) cover(d, h.tlo);
+  reset();
+  for (int64_t d = h.D - 1; d >= 0; --d) cover(d, last);
+  h.tw.assign(h.M, 0);
+  h.toff.assign(h.M, 0);
+  h.t_contiguous = true;
+  int64_t tot = 0;
+  for (int64_t i = 0; i < h.M; ++i) {
+    h.toff[i] = tot;
+    if (h.tlo[i] < 0) continue;
+    h.tw[i] = last[i] - h.tlo[i] + 1;
+    tot += h.tw[i];
+    if (h.tw[i] != h.tptr[i + 1] - h.tptr[i]) h.t_contiguous = false;
+  }
+}
+
+// Transposed CSR (ascending d per column i) where a column's d have gaps, and
+// with `bands` its band form: entries of d outside a column's CSR stay zero.
+inline void transpose_with_gaps(HostProblem& h, bool bands) {
+  const double* v = h.values();
   h.tidx.assign(h.tptr[h.M], 0);
   h.tval.assign(h.tptr[h.M], 0.0);
   std::vector<int64_t> pos(h.tptr.begin(), h.tptr.end() - 1);
@@ -171,56 +223,12 @@ inline void finish_problem(HostProblem& h) {
     for (int64_t k = 0; k < h.fw[d]; ++k) {
       const int64_t i = h.flo[d] + k;
       h.tidx[pos[i]] = (int32_t)d;
-      h.tval[pos[i]++] = h.fval[h.foff[d] + k];
+      h.tval[pos[i]++] = v[h.foff[d] + k];
     }
-  h.bdiag.assign(h.M, 0.0);
-  for (int64_t d = 0; d < h.D; ++d)
-    for (int64_t k = 0; k < h.fw[d]; ++k) {
-      const double f = h.fval[h.foff[d] + k];
-      double& b = h.bdiag[h.flo[d] + k];
-      b = b + 2.0 * (f * f);
-    }
-  if (h.gam != 0) {
-    for (int64_t j = 0; j + 1 < h.M; ++j) h.bdiag[j] = h.bdiag[j] + 2.0 * h.gam;
-    for (int64_t j = 1; j < h.M; ++j) h.bdiag[j] = h.bdiag[j] + 2.0 * h.gam;
-  }
-}
-
-// Band form of F^T from the transposed CSR: row i spans d = tidx[first] ..
-// tidx[last]; entries of d outside that row's CSR stay zero.
-inline void transposed_bands(HostProblem& h) {
-  h.tlo.assign(h.M, -1);
-  h.tw.assign(h.M, 0);
-  h.toff.assign(h.M, 0);
-  int64_t tot = 0;
-  for (int64_t i = 0; i < h.M; ++i) {
-    h.toff[i] = tot;
-    if (h.tptr[i + 1] > h.tptr[i]) {
-      h.tlo[i] = h.tidx[h.tptr[i]];
-      h.tw[i] = h.tidx[h.tptr[i + 1] - 1] - h.tlo[i] + 1;
-      tot += h.tw[i];
-    }
-  }
-  h.tbval.assign(tot, 0.0);
+  if (!bands) return;
+  h.tbval.assign(h.M > 0 ? h.toff[h.M - 1] + h.tw[h.M - 1] : 0, 0.0);
   for (int64_t i = 0; i < h.M; ++i)
     for (int64_t e = h.tptr[i]; e < h.tptr[i + 1]; ++e) h.tbval[h.toff[i] + h.tidx[e] - h.tlo[i]] = h.tval[e];
-}
-
-// Initial maxr from the seeded random X (pqdts.f90:1565-1575); call after P.
-inline std::vector<int32_t> initial_maxr(int64_t M, int64_t N, SeededStream& rng) {
-  std::vector<int32_t> mr(M);
-  std::vector<double> row(N);
-  for (int64_t i = 0; i < M; ++i) {
-    double s = 0;
-    for (int64_t n = 0; n < N; ++n) s += (row[n] = rng.next());
-    int32_t am = 0;
-    for (int64_t n = 0; n < N; ++n) {
-      row[n] = row[n] / s;
-      if (row[n] > row[am]) am = (int32_t)n;
-    }
-    mr[i] = am;
-  }
-  return mr;
 }
 
 }  // namespace pqdts

@@ -167,6 +167,29 @@ __host__ __device__ constexpr uint32_t tc_tmem_cols(int bn) {
   return bn <= 32 ? 32u : bn <= 64 ? 64u : bn <= 128 ? 128u : 256u;
 }
 
+// Band row r of F (or F^T: val[off[r] .. off[r] + w[r]) at columns lo[r] ..)
+// as a row of the tensor-core operand: hi = bf16(v), lo
+// = bf16(v - hi) at columns relative to its 128-row block's window (kb),
+// zero elsewhere.  One block per padded row.
+__global__ void __launch_bounds__(256) k_tc_split_band(const int32_t* __restrict__ lo, const int32_t* __restrict__ w,
+                                                       const int64_t* __restrict__ off,
+                                                       const double* __restrict__ val,
+                                                       const int32_t* __restrict__ kb, int R, int kmax,
+                                                       __nv_bfloat16* __restrict__ hi,
+                                                       __nv_bfloat16* __restrict__ low) {
+  const int r = blockIdx.x;
+  const int width = r < R ? w[r] : 0;
+  const int start = width > 0 ? lo[r] - kb[r / kTcRows] : 0;
+  const double* v = val + (width > 0 ? off[r] : 0);
+  for (int x = threadIdx.x; x < kmax; x += blockDim.x) {
+    const int k = x - start;
+    const double y = (unsigned)k < (unsigned)width ? v[k] : 0.0;
+    const __nv_bfloat16 h = __double2bfloat16(y);
+    hi[(int64_t)r * kmax + x] = h;
+    low[(int64_t)r * kmax + x] = __double2bfloat16(y - (double)__bfloat162float(h));
+  }
+}
+
 // mode 0: FP32 Out[z * out_stride + r * N + n] = scale * acc (row-major; z =
 //         the K split whose partial this is).
 // mode 1: Out^T split again: oh[n * ld + r] = hi, ol[n * ld + r] = lo of
