@@ -48,8 +48,10 @@ const double kHuge = std::numeric_limits<double>::max();
 constexpr int kMaxCG = 50;                 // do j = 1, 50 (2036)
 constexpr int kMaxLS = 100;                // do i = 1, 100 (374, 420, 466)
 constexpr int kBatchLS = 8;                // step lengths evaluated per sweep
+constexpr int64_t kPinnedRows = 4096;       // simplexproj calls of up to this many values go through pinned memory
+constexpr int64_t kProjKeep = 1 << 25;      // ... and of up to this many keep their device rows for the next one
 constexpr int kElemGrid = 152 * 8;         // elementwise grids: 8 blocks per SM
-constexpr size_t kCondatSmemMax = 200u * 1024u;  // Condat's rows staged in shared memory up to this size
+constexpr size_t kRowSmemMax = 200u * 1024u;  // k_simplex_smem's rows staged in shared memory up to this size
 
 struct Err : std::runtime_error {
   int code;
@@ -406,6 +408,10 @@ struct pqdts_ctx {
   pqdts::DBuf<int> ipart;
   pqdts::DBuf<long long> icount;
   double* pin = nullptr;  // pinned host scalars
+  // simplexproj's rows: on the device (kept between calls up to kProjKeep
+  // values) and, for small calls, pinned (allocated on first use)
+  pqdts::DBuf<double> proj;
+  double* proj_pin = nullptr;
   bool fullspace = true;
   std::vector<int32_t> h_maxr;
   pqdts::GpuTimers timers;
@@ -798,8 +804,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
   }
   c.fmacount.alloc(2);
   CK(cudaMemsetAsync(c.fmacount.p, 0, 2 * sizeof(unsigned long long), c.st));
-  CK(cudaFuncSetAttribute(k_condat_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCondatSmemMax));
-  CK(cudaFuncSetAttribute(k_simplex_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCondatSmemMax));
+  CK(cudaFuncSetAttribute(k_simplex_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmemMax));
   c.counters.alloc(8);
   CK(cudaMemsetAsync(c.counters.p, 0, 8 * sizeof(unsigned), c.st));
   c.exact = (c.precision == PQDTS_FP64);
@@ -1994,6 +1999,15 @@ static void cg_solve(Ctx& c, CGBufs<T>& b, const T* fv, const T* tv, double bdfa
   }
 }
 
+// k_condat over B stacked sets of M rows: one row a warp until every SM
+// sub-partition of the GPU (152 SMs x 4) has a warp, then more rows a warp.
+static void launch_condat(const double* X, const double* S, const double* alphas, double* out, double* aux,
+                          int64_t stride, int M, int N, int B, cudaStream_t st) {
+  const int RP = (int)std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)M * B + 607) / 608));
+  k_condat<<<dim3(cdiv(M, RP * kCondatWarps), B), 32 * kCondatWarps, 0, st>>>(X, S, alphas, out, aux, stride, M, N,
+                                                                              RP);
+}
+
 // Row-wise simplex projection (doproj, 1120-1140) of X + alpha_b*S (or of X
 // when S is null) into out[b].  FP64 path: Condat's algorithm in the
 // reference's order (bitwise equal to condat_simplexproj.c), one thread per
@@ -2002,16 +2016,11 @@ static void project_rows(Ctx& c, const double* X, const double* S, const double*
   const int M = (int)c.h.M, N = (int)c.h.N;
   const int64_t MN = (int64_t)M * N;
   if (c.exact) {
-    const size_t smem = (size_t)2 * 33 * N * sizeof(double);
-    if (smem <= kCondatSmemMax) {
-      k_condat_smem<<<dim3(cdiv(M, 32), B), 32, smem, c.st>>>(X, S, alphas, out, MN, M, N);
-    } else {
-      require(c.aux.p, "aux");
-      k_condat<<<dim3(cdiv(M, kRowThreads), B), kRowThreads, 0, c.st>>>(X, S, alphas, out, c.aux.p, MN, M, N);
-    }
+    require(c.aux.p, "aux");
+    launch_condat(X, S, alphas, out, c.aux.p, MN, M, N, B, c.st);
   } else {
     // rows staged in shared memory: up to 4 warps (rows) per block
-    const int wpb = (int)std::min<int64_t>(4, (int64_t)kCondatSmemMax / ((int64_t)N * 8));
+    const int wpb = (int)std::min<int64_t>(4, (int64_t)kRowSmemMax / ((int64_t)N * 8));
     if (wpb >= 1) {
       k_simplex_smem<<<dim3(cdiv(M, wpb), B), 32 * wpb, (size_t)wpb * N * sizeof(double), c.st>>>(X, S, alphas, out,
                                                                                                  MN, M, N);
@@ -3191,6 +3200,7 @@ int pqdts_cuda_destroy(pqdts_ctx* c) {
   cudaSetDevice(c->device);
   if (c->st) cudaStreamSynchronize(c->st);
   if (c->pin) cudaFreeHost(c->pin);
+  if (c->proj_pin) cudaFreeHost(c->proj_pin);
   cudaStream_t st = c->own_stream ? c->st : nullptr;
   delete c;
   if (st) cudaStreamDestroy(st);
@@ -3461,15 +3471,27 @@ int pqdts_cuda_simplexproj(pqdts_ctx* c, const double* y, double* x, int64_t len
   return guarded(c, [&] {
     if (!y || !x || len <= 0 || rows <= 0) throw Err(PQDTS_E_ARG, "bad simplexproj arguments");
     if (len * rows >= ((int64_t)1 << 31)) throw Err(PQDTS_E_ARG, "simplexproj input too large");
-    pqdts::DBuf<double> d, w;
-    d.alloc((size_t)(len * rows));
-    w.alloc((size_t)(len * rows));
-    CK(cudaMemcpyAsync(d.p, y, len * rows * 8, cudaMemcpyHostToDevice, c->st));
-    pqdts::k_condat<<<dim3(pqdts::cdiv(rows, pqdts::kRowThreads), 1), pqdts::kRowThreads, 0, c->st>>>(
-        d.p, nullptr, nullptr, d.p, w.p, 0, (int)rows, (int)len);
+    const int64_t n = len * rows;
+    if (n <= pqdts::kPinnedRows) {
+      // small calls are all fixed cost: the rows go through pinned memory
+      // that the kernel reads and writes itself, one launch and no copies
+      if (!c->proj_pin) CK(cudaMallocHost((void**)&c->proj_pin, pqdts::kPinnedRows * sizeof(double)));
+      c->proj.alloc(pqdts::kPinnedRows);
+      std::memcpy(c->proj_pin, y, n * sizeof(double));
+      pqdts::launch_condat(c->proj_pin, nullptr, nullptr, c->proj_pin, c->proj.p, 0, (int)rows, (int)len, 1, c->st);
+      pqdts::post_launch(*c);
+      CK(cudaStreamSynchronize(c->st));
+      std::memcpy(x, c->proj_pin, n * sizeof(double));
+      return;
+    }
+    c->proj.alloc((size_t)(2 * n));
+    double* d = c->proj.p;
+    CK(cudaMemcpyAsync(d, y, n * 8, cudaMemcpyHostToDevice, c->st));
+    pqdts::launch_condat(d, nullptr, nullptr, d, d + n, 0, (int)rows, (int)len, 1, c->st);
     pqdts::post_launch(*c);
-    CK(cudaMemcpyAsync(x, d.p, len * rows * 8, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(x, d, n * 8, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (n > pqdts::kProjKeep) c->proj.release();
   });
 }
 
@@ -3527,7 +3549,7 @@ void simplexproj_condat_(double* y, double* x, int* plength) {
   double* d = t.buf;
   double* w = t.buf + t.cap;
   if ((e = cudaMemcpyAsync(d, y, (size_t)len * 8, cudaMemcpyHostToDevice, t.st)) != cudaSuccess) return fail("upload");
-  pqdts::k_condat<<<1, 32, 0, t.st>>>(d, nullptr, nullptr, d, w, 0, 1, len);
+  pqdts::launch_condat(d, nullptr, nullptr, d, w, 0, 1, len, 1, t.st);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail("launch");
   if ((e = cudaMemcpyAsync(x, d, (size_t)len * 8, cudaMemcpyDeviceToHost, t.st)) != cudaSuccess) return fail("download");
   if ((e = cudaStreamSynchronize(t.st)) != cudaSuccess) return fail("projection");
@@ -3605,8 +3627,7 @@ int pqdts_cuda_simplexproj_noalloc(const double* d_y, double* d_x, int64_t len, 
     }
     scratch = slot.ptr;
   }
-  pqdts::k_condat<<<dim3(pqdts::cdiv(rows, pqdts::kRowThreads), 1), pqdts::kRowThreads, 0, (cudaStream_t)stream>>>(
-      d_y, nullptr, nullptr, d_x, scratch, 0, (int)rows, (int)len);
+  pqdts::launch_condat(d_y, nullptr, nullptr, d_x, scratch, 0, (int)rows, (int)len, 1, (cudaStream_t)stream);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     fprintf(stderr, "pqdts_cuda_simplexproj_noalloc: launch failed: %s\n", cudaGetErrorString(e));
