@@ -422,6 +422,16 @@ struct pqdts_ctx {
   double target_L = 0.0;  // optional objective stopping rule (0 = off)
   // version of X, bumped on every write; results keyed on it are reused
   int64_t xver = 0, R_ver = -1, G_ver = -1, L_ver = -1, rebuilt_ver = -1;
+  // FP64 path: most versions of X are max-column rebuilds of the last one,
+  // which move an ulp of a few rows.  Their columns are recorded -- chg[n]
+  // since R was formed, chg[N + n] since the raw sums F^T.R in Graw were -- and
+  // only those are formed again; xfull is the last version that changed X in
+  // any other way, saved the entries behind the stage-2 placeholders
+  // (placeholder: those are in X now).
+  pqdts::DBuf<int32_t> chg;
+  pqdts::DBuf<double> Graw, saved;
+  int64_t xfull = 0, Graw_ver = -1;
+  bool placeholder = false;
   bool G_full = true;
   double L_cache = 0.0, Lgam_cache = 0.0;  // L of X (version L_ver) and its gamma term
   bool target_hit = false;
@@ -534,7 +544,10 @@ static DevBands bands_of(Ctx& c) {
 static inline int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // X changed: results keyed on the old version are stale.
-static void touch_x(Ctx& c) { c.xver++; }
+static void touch_x(Ctx& c) {
+  c.xfull = ++c.xver;
+  c.placeholder = false;
+}
 
 static void post_launch(Ctx& c) {
   c.launches++;
@@ -563,7 +576,7 @@ static void throw_tc_error(Ctx& c) {
   CK(cudaMemsetAsync(c.sc.p + SC_TCERR, 0, sizeof(double), c.st));
   CK(cudaStreamSynchronize(c.st));
   // what the product was to write is not there
-  c.R_ver = c.G_ver = c.Gf_ver = c.L_ver = -1;
+  c.R_ver = c.G_ver = c.Gf_ver = c.L_ver = c.Graw_ver = -1;
   throw Err(PQDTS_E_CUDA, "tensor-core product: a barrier wait timed out");
 }
 
@@ -819,6 +832,15 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
   c.lred.alloc(kBatchLS);
   c.X.alloc(MN);
   c.G.alloc(MN);
+  if (c.exact) {
+    c.chg.alloc(2 * N);
+    c.saved.alloc(M);
+    c.Graw.alloc(MN);
+  } else {
+    c.chg.release();
+    c.saved.release();
+    c.Graw.release();
+  }
   c.Xc.alloc((size_t)kBatchLS * MN);
   c.R.alloc(D * N);
   c.sn64.alloc(MN);
@@ -836,7 +858,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
   // Initial X = 1/N (pqdts.f90:1834-1838) and maxr from the seeded stream.
   k_fill<<<elem_grid(MN), 256, 0, c.st>>>(MN, 1.0 / (double)N, c.X.p);
   post_launch(c);
-  c.R_ver = c.G_ver = c.L_ver = c.rebuilt_ver = c.Gf_ver = -1;
+  c.R_ver = c.G_ver = c.L_ver = c.rebuilt_ver = c.Gf_ver = c.Graw_ver = -1;
   touch_x(c);
   CK(cudaStreamSynchronize(c.st));
   c.fullspace = true;
@@ -850,9 +872,9 @@ static void need_problem(Ctx& c) {
 // ---------------------------------------------------------------------------
 // Operations on device arrays.
 // ---------------------------------------------------------------------------
-static void rebuild(Ctx& c, double* X, int B = 1) {
+static void rebuild(Ctx& c, double* X, const double* saved, int32_t* chg) {
   const int M = (int)c.h.M, N = (int)c.h.N;
-  k_rebuild_t<<<dim3(cdiv(M, 32), B), kTileThreads, 0, c.st>>>(X, (int64_t)M * N, c.maxr.p, M, N);
+  k_rebuild_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(X, (int64_t)M * N, c.maxr.p, M, N, saved, chg);
   post_launch(c);
 }
 
@@ -911,10 +933,12 @@ static int rows_per_block(int N) {
 }
 
 // F.X (B stacked inputs, xstride apart) with the epilogue MODE of k_fwd, in
-// the context's form: column-tiled, or row-flattened (rows = 1; the same bits).
+// the context's form: column-tiled, or row-flattened (rows = 1; the same
+// bits).  cols != null: only those columns need forming (B = 1; the forms
+// without column lists form all).
 template <typename T, int MODE>
 static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const double* P, T* R, int B,
-                       const double* pred, int rows = -1) {
+                       const double* pred, int rows = -1, const int32_t* cols = nullptr) {
   const int N = (int)c.h.N, D = (int)c.h.D;
   DevBands bd = bands_of(c);
   const int RB = rows_per_block(N);
@@ -924,11 +948,11 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
       // X where X[i, n] != 0 (X's column lists; the same bits)
       const int M = (int)c.h.M;
       k_col_index<T><<<dim3(cdiv(N, kIndexWarps), B), 32 * kIndexWarps, 0, c.st>>>(X, xstride, M, N, c.xcmask.p,
-                                                                                  c.xccnt.p, c.xclist.p);
+                                                                                  c.xccnt.p, c.xclist.p, cols);
       post_launch(c);
       k_fwd_col<T, MODE><<<dim3(cdiv(N, kTcWarps), cdiv(D, 32), B), dim3(32, kTcWarps), 0, c.st>>>(
           M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride, c.xcmask.p, c.xccnt.p,
-          c.xclist.p, P, R, pred, c.count_fmas ? c.fmacount.p : nullptr);
+          c.xclist.p, P, R, pred, c.count_fmas ? c.fmacount.p : nullptr, cols);
       post_launch(c);
       return;
     }
@@ -1035,14 +1059,29 @@ static void fetch_objectives(Ctx& c, int B, double* L) {
 
 // Max-column rebuild of the context's X.  FP64 path: always a new version
 // of X (across M rows some row practically always moves by an ulp, and the
-// trajectory must stay bit-exact).  Mixed path: re-applying the rebuild to
-// an X that is already consistent with maxr only moves values by ulps, so
-// results computed for that X stay in use.
+// trajectory must stay bit-exact), with the columns that moved recorded.
+// Mixed path: re-applying the rebuild to an X that is already consistent with
+// maxr only moves values by ulps, so results computed for that X stay in use.
 static void rebuild_x(Ctx& c) {
-  rebuild(c, c.X.p);
-  if (!c.exact && c.rebuilt_ver == c.xver) return;
+  if (c.exact) {
+    rebuild(c, c.X.p, c.placeholder ? c.saved.p : nullptr, c.chg.p);
+    c.xver++;  // not touch_x: this change is on record
+    c.placeholder = false;
+    return;
+  }
+  rebuild(c, c.X.p, nullptr, nullptr);
+  if (c.rebuilt_ver == c.xver) return;
   touch_x(c);
   c.rebuilt_ver = c.xver;
+}
+
+// The columns to form again (chg's first or second half) for a result of
+// version `ver` of X, or null: all of them.
+static const int32_t* changed_columns(Ctx& c, int64_t ver, int half) {
+  return c.exact && ver >= 0 && ver >= c.xfull ? c.chg.p + half * c.h.N : nullptr;
+}
+static void clear_changed(Ctx& c, int half) {
+  if (c.exact) CK(cudaMemsetAsync(c.chg.p + half * c.h.N, 0, c.h.N * sizeof(int32_t), c.st));
 }
 
 // R = 2*(O - P) with O = F.X for the context's X, unless R already holds it
@@ -1050,7 +1089,9 @@ static void rebuild_x(Ctx& c) {
 static void ensure_R(Ctx& c) {
   if (c.R_ver == c.xver) return;
   if (c.df_fwd) fwd_df<0>(c, c.X.p, c.R.p);
-  else launch_fwd<double, 0>(c, c.fval.p, c.X.p, 0, c.P.p, c.R.p, 1, nullptr);
+  else
+    launch_fwd<double, 0>(c, c.fval.p, c.X.p, 0, c.P.p, c.R.p, 1, nullptr, -1, changed_columns(c, c.R_ver, 0));
+  clear_changed(c, 0);
   c.R_ver = c.xver;
 }
 
@@ -1100,32 +1141,36 @@ static TransShape trans_shape(int N) {
   return best;
 }
 
+// (sums: where the column form keeps its sums before the epilogue, G itself
+// unless given; cols != null: only those columns' sums need forming, the
+// others are in `sums`.)
 // k_trans with an explicit block shape (every shape gives the same values:
 // each output accumulates its CSR row in ascending order in one thread).
 template <typename T, bool HVP>
 static void launch_trans_shape(Ctx& c, TransShape sh, const T* tv, const T* R, const T* V, const T* rs, int reduced,
                                T c2gam, const int8_t* ik, T* G, const T* W, double* dpart, const double* pred,
-                               T* Gf = nullptr) {
+                               T* Gf = nullptr, T* sums = nullptr, const int32_t* cols = nullptr) {
   const int M = (int)c.h.M;
   DevBands bd = bands_of(c);
   const int RB = rows_per_block((int)c.h.N);
-  int raw = 0;
+  const T* raw = nullptr;
   if constexpr (std::is_same<T, double>::value) {
     if (c.mask_option != 0 && c.ftile.p != nullptr && tv == c.tval.p) {
       // FP64: the sums by (column n, 32-row tile of F^T) warps visiting only
       // the d where R[d, n] != 0 (R's column lists; the same bits), then
       // k_trans's epilogue on them
       const int N = (int)c.h.N, D = (int)c.h.D;
+      T* acc = sums ? sums : G;
       k_col_index<T><<<cdiv(N, kIndexWarps), 32 * kIndexWarps, 0, c.st>>>(R, 0, D, N, c.rmask.p, c.ccnt.p,
-                                                                          c.clist.p);
+                                                                          c.clist.p, cols);
       post_launch(c);
       // with the active set (the CG's product), warps whose outputs are all
       // masked by the epilogue skip their sums
       k_trans_col<T><<<dim3(cdiv(N, kTcWarps), cdiv(M, 32)), dim3(32, kTcWarps), 0, c.st>>>(
-          M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, G, pred,
-          c.count_fmas ? c.fmacount.p + 1 : nullptr, ik, reduced ? c.maxr.p : nullptr);
+          M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, acc, pred,
+          c.count_fmas ? c.fmacount.p + 1 : nullptr, ik, reduced ? c.maxr.p : nullptr, cols);
       post_launch(c);
-      raw = 1;
+      raw = acc;
     }
   }
   if (raw) {
@@ -1160,11 +1205,12 @@ static void launch_trans_shape(Ctx& c, TransShape sh, const T* tv, const T* R, c
 // k_trans with the context's schedule.
 template <typename T, bool HVP>
 static void launch_trans(Ctx& c, const T* tv, const T* R, const T* V, const T* rs, int reduced, T c2gam,
-                         const int8_t* ik, T* G, const T* W, double* dpart, const double* pred, T* Gf = nullptr) {
+                         const int8_t* ik, T* G, const T* W, double* dpart, const double* pred, T* Gf = nullptr,
+                         T* sums = nullptr, const int32_t* cols = nullptr) {
   TransShape sh = c.sched.trans_threads > 0 ? TransShape{c.sched.trans_threads, c.sched.trans_cols}
                                             : trans_shape((int)c.h.N);
   sh.rows = c.sched.trans_rows;
-  launch_trans_shape<T, HVP>(c, sh, tv, R, V, rs, reduced, c2gam, ik, G, W, dpart, pred, Gf);
+  launch_trans_shape<T, HVP>(c, sh, tv, R, V, rs, reduced, c2gam, ik, G, W, dpart, pred, Gf, sums, cols);
 }
 
 // dL(X) -> c.G (975-1032), reusing R and the gradient itself when X and the
@@ -1213,8 +1259,12 @@ static void op_dL(Ctx& c) {
     ensure_R(c);
     double* gf = (!c.exact && !c.fullspace) ? c.Gf.p : nullptr;
     launch_trans<double, false>(c, c.tval.p, c.R.p, c.X.p, nullptr, c.fullspace ? 0 : 1, 2.0 * c.h.gam, nullptr,
-                                c.G.p, nullptr, nullptr, nullptr, gf);
-    if (!c.exact) {
+                                c.G.p, nullptr, nullptr, nullptr, gf, c.exact ? c.Graw.p : nullptr,
+                                changed_columns(c, c.Graw_ver, 1));
+    if (c.exact) {
+      clear_changed(c, 1);
+      c.Graw_ver = c.mask_option != 0 && c.ftile.p != nullptr ? c.xver : -1;  // only the column form leaves sums
+    } else {
       if (c.fullspace) CK(cudaMemcpyAsync(c.Gf.p, c.G.p, (size_t)M * N * 8, cudaMemcpyDeviceToDevice, c.st));
       c.Gf_ver = c.xver;
     }
@@ -2316,10 +2366,13 @@ static double outer_pre_cg(Ctx& c, int oiter) {
   const int M = (int)c.h.M, N = (int)c.h.N;
   c.fullspace = (oiter == 1);
   if (!c.fullspace) {
-    k_stage2_start_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(c.X.p, c.maxr.p, M, N, 1);
+    k_stage2_start_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(c.X.p, c.maxr.p, M, N, 1,
+                                                             c.exact ? c.saved.p : nullptr,
+                                                             c.exact ? c.chg.p : nullptr);
     post_launch(c);
     if (c.exact) {
-      touch_x(c);
+      c.xver++;  // on record: the rebuild's columns, and the placeholders' entries
+      c.placeholder = true;
     } else {
       // mixed path: the placeholder is replaced by the next rebuild, which
       // restores X to within ulps; only the reduced gradient (new maxr)
@@ -2389,11 +2442,14 @@ static void outer_tail(Ctx& c, SolveState& st) {
   const int M = (int)c.h.M, N = (int)c.h.N;
   const int64_t MN = (int64_t)M * N;
   const int g = elem_grid(MN);
-  // Mixed path: the chosen step was evaluated to FP64 accuracy as a
-  // line-search candidate (projected, rebuilt, its residual and objective known): adopt
-  // it instead of recomputing the same projection and banded product.
+  // The chosen step was evaluated as a line-search candidate (projected,
+  // rebuilt as L does, its residual and objective known; FP64 path: by the
+  // same operations on the same operands as below, so the same bits; mixed
+  // path: to FP64 accuracy): while it is still in the candidates' stack,
+  // adopt it instead of computing the projection, the banded product and the
+  // objective's sums once more.
   int adopt = -1;
-  if (!c.exact && st.alpha != 0.0 && c.cand_xver == c.xver && c.cand_stage2 == !c.fullspace)
+  if (st.alpha != 0.0 && c.cand_xver == c.xver && c.cand_stage2 == !c.fullspace)
     for (int b = 0; b < c.cand_B; ++b)
       if (c.cand_alpha[b] == st.alpha) {
         adopt = b;
@@ -2407,6 +2463,7 @@ static void outer_tail(Ctx& c, SolveState& st) {
     k_scale_copy<<<elem_grid(DN), 256, 0, c.st>>>(DN, 2.0, c.Rst.p + (size_t)adopt * DN, c.R.p);
     post_launch(c);
     c.R_ver = c.xver;
+    clear_changed(c, 0);
     c.L_cache = c.cand_L[adopt];
     c.Lgam_cache = c.cand_Lgam[adopt];
     c.L_ver = c.xver;
@@ -2436,7 +2493,9 @@ static void outer_tail(Ctx& c, SolveState& st) {
     read_back(c, c.sc.p + SC_TMP, 1);
     st.xmin = c.pin[0];
   }
-  st.L0 = op_L(c);
+  // (the adopted candidate has had L's rebuild; FP64 path: one more would be
+  // one too many)
+  st.L0 = c.exact && adopt >= 0 ? c.L_cache : op_L(c);
   op_dL(c);
   // |der|^2 of this space's gradient, read back with conv_test's value
   dot_dev(c, c.G.p, c.G.p, c.sc.p + SC_TMP + 1);
