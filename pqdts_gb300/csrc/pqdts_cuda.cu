@@ -878,6 +878,27 @@ static void rebuild(Ctx& c, double* X, const double* saved, int32_t* chg) {
   post_launch(c);
 }
 
+// Column chains (k_colchain's OP) of B stacked inputs: a block a chain while
+// that leaves an SM at most two blocks and the chain is long enough to pay
+// for the guess (two chains of 1000 terms a column, 200 blocks: 39 us either
+// way; one: 29 against 39 by warps, 22 against 19 at 200 terms), a warp a
+// chain otherwise.
+template <int OP>
+static void launch_colchain(Ctx& c, const double* a, const double* b, int64_t stride, int B, double* out, double* out2,
+                            const double* pred, double* sum_out, int ostride, unsigned* counter) {
+  const int M = (int)c.h.M, N = (int)c.h.N;
+  const int chains = N * (OP == 2 ? 2 : 1);
+  if (M >= (OP == 2 ? 1500 : 500) && (int64_t)chains * B <= (OP == 2 ? 3 : 2) * 152) {
+    k_colchain_b<OP><<<dim3(chains, B), 32 * kBcWarps, 0, c.st>>>(a, b, stride, M, N, c.h.gam, out, out2, pred, sum_out,
+                                                                  ostride, counter);
+  } else {
+    constexpr int per = OP == 2 ? kChainWarps / 2 : kChainWarps;
+    k_colchain<OP><<<dim3(cdiv(N, per), B), 32 * kChainWarps, 0, c.st>>>(a, b, stride, M, N, c.h.gam, out, out2, pred,
+                                                                         sum_out, ostride, counter);
+  }
+  post_launch(c);
+}
+
 // Objective from the per-row residual sums srow[b][d] of B matrices Xs
 // (L_red) plus the gamma term of Xs (L_gam, 954-964) -> lsout[b].  FP64 path:
 // rows added in ascending order, then the gamma term's column chains added
@@ -889,9 +910,7 @@ static void objective_combine(Ctx& c, const double* Xs, int B) {
     k_seqsum<<<B, 32, 0, c.st>>>(c.srow.p, D, nullptr, out, B, nullptr);
     post_launch(c);
     if (c.h.gam != 0) {
-      k_colchain<1><<<dim3(cdiv(N, kChainWarps), B), 32 * kChainWarps, 0, c.st>>>(
-          Xs, nullptr, (int64_t)M * N, M, N, c.h.gam, c.gcol.p, nullptr, nullptr);
-      post_launch(c);
+      launch_colchain<1>(c, Xs, nullptr, (int64_t)M * N, B, c.gcol.p, nullptr, nullptr, nullptr, 1, nullptr);
       k_seqsum<<<B, 32, 0, c.st>>>(c.gcol.p, N, c.lred.p, c.lsout.p, B, nullptr);
       post_launch(c);
     }
@@ -1276,15 +1295,12 @@ static void op_dL(Ctx& c) {
 // pdot (589-614): sum(a.b) over M*N -> device scalar `out`.  FP64 path: one
 // chain per column over the rows, columns added in ascending order.
 static void dot_dev(Ctx& c, const double* a, const double* b, double* out, const double* pred = nullptr) {
-  const int M = (int)c.h.M, N = (int)c.h.N;
   if (c.exact) {
     // column chains, then (last block) their ascending sum into out
-    k_colchain<0><<<dim3(cdiv(N, kChainWarps), 1), 32 * kChainWarps, 0, c.st>>>(a, b, 0, M, N, 0.0, c.colbuf.p,
-                                                                                nullptr, pred, out, 1, c.counters.p + 2);
-    post_launch(c);
+    launch_colchain<0>(c, a, b, 0, 1, c.colbuf.p, nullptr, pred, out, 1, c.counters.p + 2);
     return;
   }
-  const int64_t total = (int64_t)M * N;
+  const int64_t total = c.h.M * c.h.N;
   const int g = elem_grid(total);
   k_dot_part<<<g, 256, 0, c.st>>>(total, a, b, c.part.p);
   post_launch(c);
@@ -1295,10 +1311,7 @@ static void dot_dev(Ctx& c, const double* a, const double* b, double* out, const
 // out_aa = out_ab + ostride (a warp per chain, two per column).
 static void dot2_exact(Ctx& c, const double* a, const double* b, double* out_ab, int ostride,
                        const double* pred) {
-  const int M = (int)c.h.M, N = (int)c.h.N;
-  k_colchain<2><<<dim3(cdiv(N, kChainWarps / 2), 1), 32 * kChainWarps, 0, c.st>>>(
-      a, b, 0, M, N, 0.0, c.colbuf.p, c.colbuf.p + N, pred, out_ab, ostride, c.counters.p + 3);
-  post_launch(c);
+  launch_colchain<2>(c, a, b, 0, 1, c.colbuf.p, c.colbuf.p + c.h.N, pred, out_ab, ostride, c.counters.p + 3);
 }
 
 // Hessian-vector product of one precision: Hp = H p (BF, 246-342); masks the
