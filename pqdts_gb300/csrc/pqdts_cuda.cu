@@ -846,7 +846,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
   c.sn64.alloc(MN);
   c.ik.alloc(MN);
   const int64_t fwd_parts = (int64_t)cdiv(N, kBX) * cdiv(D, kBY) * kBatchLS;
-  const int64_t np = std::max<int64_t>({fwd_parts, M, (int64_t)kElemGrid * kBatchLS, 1024});
+  const int64_t np = std::max<int64_t>({fwd_parts, M, (int64_t)kBatchLS * cdiv(M, kRowWarps), (int64_t)kElemGrid * kBatchLS, 1024});
   c.part.alloc(np);
   c.part2.alloc(np);
   c.icount.alloc(1);
@@ -1056,6 +1056,34 @@ static void fwd_df(Ctx& c, const double* X, double* R) {
   launch_fwd_df<MODE>(c, R, xm);
 }
 
+// Residual row sums of B stacked residuals, each scale * R, into srow.
+static void residual_rows(Ctx& c, const double* R, double scale, int B) {
+  const int D = (int)c.h.D, N = (int)c.h.N;
+  if (c.exact)
+    k_rowchain_resid_t<<<dim3(cdiv(D, 32), B), kTileThreads, 0, c.st>>>(R, c.flo.p, D, N, scale, c.srow.p);
+  else
+    k_rowresid_w<<<dim3(cdiv(D, kRowWarps), B), 32 * kRowWarps, 0, c.st>>>(R, c.flo.p, D, N, scale, c.srow.p);
+  post_launch(c);
+}
+
+// Reduced-space candidates Xc[b] = X + alpha_b S (or, S null, Xc[0] itself)
+// clipped and rebuilt (doproj2, 1142-1164), with l_rebuild also the rebuild
+// that L performs on entry; their smallest max-column entries (at most 0)
+// into xmin[0 .. B).
+static void candidates_proj2(Ctx& c, const double* X, const double* S, double* Xc, int B, int l_rebuild,
+                             double* xmin) {
+  const int M = (int)c.h.M, N = (int)c.h.N;
+  const int64_t MN = (int64_t)M * N;
+  const int gb = cdiv(M, c.exact ? 32 : kRowWarps);  // 32-row tiles, or a warp a row
+  if (c.exact)
+    k_cand_proj2_t<<<dim3(gb, B), kTileThreads, 0, c.st>>>(X, S, c.alphas.p, Xc, MN, c.maxr.p, M, N, l_rebuild,
+                                                           c.part2.p);
+  else
+    k_cand_proj2_w<<<dim3(gb, B), 32 * kRowWarps, 0, c.st>>>(X, S, c.alphas.p, Xc, MN, c.maxr.p, M, N, c.part2.p);
+  post_launch(c);
+  reduce_to(c, c.part2.p, gb, xmin, B, true, 0.0);
+}
+
 static void objective_stack(Ctx& c, const double* Xs, int B) {
   const int M = (int)c.h.M, N = (int)c.h.N, D = (int)c.h.D;
   require(c.Rst.p, "Rst");
@@ -1065,8 +1093,7 @@ static void objective_stack(Ctx& c, const double* Xs, int B) {
   } else {
     launch_fwd<double, 3>(c, c.fval.p, Xs, (int64_t)M * N, c.P.p, c.Rst.p, B, nullptr);
   }
-  k_rowchain_resid_t<<<dim3(cdiv(D, 32), B), kTileThreads, 0, c.st>>>(c.Rst.p, c.flo.p, D, N, 1.0, c.srow.p);
-  post_launch(c);
+  residual_rows(c, c.Rst.p, 1.0, B);
   objective_combine(c, Xs, B);
 }
 
@@ -1088,7 +1115,8 @@ static void rebuild_x(Ctx& c) {
     c.placeholder = false;
     return;
   }
-  rebuild(c, c.X.p, nullptr, nullptr);
+  k_rebuild_w<<<cdiv(c.h.M, kRowWarps), 32 * kRowWarps, 0, c.st>>>(c.X.p, c.maxr.p, (int)c.h.M, (int)c.h.N);
+  post_launch(c);
   if (c.rebuilt_ver == c.xver) return;
   touch_x(c);
   c.rebuilt_ver = c.xver;
@@ -1122,8 +1150,7 @@ static double op_L(Ctx& c) {
   if (c.L_ver == c.xver) return c.L_cache;
   ensure_R(c);
   const int D = (int)c.h.D, N = (int)c.h.N;
-  k_rowchain_resid_t<<<dim3(cdiv(D, 32), 1), kTileThreads, 0, c.st>>>(c.R.p, c.flo.p, D, N, 0.5, c.srow.p);
-  post_launch(c);
+  residual_rows(c, c.R.p, 0.5, 1);
   objective_combine(c, c.X.p, 1);
   double L;
   fetch_objectives(c, 1, &L);
@@ -2101,12 +2128,8 @@ static void eval_candidates(Ctx& c, const double* al, int B, bool stage2, double
   const int64_t MN = (int64_t)M * N;
   CK(cudaMemcpyAsync(c.alphas.p, al, B * sizeof(double), cudaMemcpyHostToDevice, c.st));
   if (stage2) {
-    const int gb = cdiv(M, 32);  // 32-row tiles
     Scope s(c.timers, "doproj2");
-    k_cand_proj2_t<<<dim3(gb, B), kTileThreads, 0, c.st>>>(c.X.p, c.sn64.p, c.alphas.p, c.Xc.p, MN, c.maxr.p, M, N, 1,
-                                                         c.part2.p);
-    post_launch(c);
-    reduce_to(c, c.part2.p, gb, c.lsout.p + 2 * kBatchLS, B, true, 0.0);
+    candidates_proj2(c, c.X.p, c.sn64.p, c.Xc.p, B, 1, c.lsout.p + 2 * kBatchLS);
   } else {
     Scope s(c.timers, "doproj");
     project_rows(c, c.X.p, c.sn64.p, c.alphas.p, c.Xc.p, B);
@@ -2227,11 +2250,7 @@ static void line_search_mixed(Ctx& c, bool stage2, double& alpha, double& dlalph
   auto screen = [&](const double* qa, int nb, double* dL, double* xmin) {
     CK(cudaMemcpyAsync(c.alphas.p, qa, nb * sizeof(double), cudaMemcpyHostToDevice, c.st));
     if (stage2) {
-      const int gb = cdiv(M, 32);  // 32-row tiles
-      k_cand_proj2_t<<<dim3(gb, nb), kTileThreads, 0, c.st>>>(c.X.p, c.sn64.p, c.alphas.p, c.Xc.p, MN, c.maxr.p, M, N, 1,
-                                                            c.part2.p);
-      post_launch(c);
-      reduce_to(c, c.part2.p, gb, c.lsout.p + 2 * kBatchLS, nb, true, 0.0);
+      candidates_proj2(c, c.X.p, c.sn64.p, c.Xc.p, nb, 1, c.lsout.p + 2 * kBatchLS);
     } else {
       project_rows(c, c.X.p, c.sn64.p, c.alphas.p, c.Xc.p, nb);
     }
@@ -2330,8 +2349,11 @@ static double op_conv(Ctx& c, bool tprint, bool with_extra = false) {
   op_dL(c);
   DBuf<double> lam;
   if (tprint && c.verbose) lam.alloc(M);
-  k_conv_rows_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(c.X.p, c.G.p, M, N, c.part.p,
-                                                        (tprint && c.verbose) ? lam.p : nullptr);
+  double* lam_out = (tprint && c.verbose) ? lam.p : nullptr;
+  if (c.exact)
+    k_conv_rows_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(c.X.p, c.G.p, M, N, c.part.p, lam_out);
+  else
+    k_conv_rows_w<<<cdiv(M, kRowWarps), 32 * kRowWarps, 0, c.st>>>(c.X.p, c.G.p, M, N, c.part.p, lam_out);
   post_launch(c);
   if (c.exact) {
     k_seqsum<<<1, 32, 0, c.st>>>(c.part.p, M, nullptr, c.sc.p + SC_TMP, 1, nullptr);
@@ -2379,9 +2401,10 @@ static double outer_pre_cg(Ctx& c, int oiter) {
   const int M = (int)c.h.M, N = (int)c.h.N;
   c.fullspace = (oiter == 1);
   if (!c.fullspace) {
-    k_stage2_start_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(c.X.p, c.maxr.p, M, N, 1,
-                                                             c.exact ? c.saved.p : nullptr,
-                                                             c.exact ? c.chg.p : nullptr);
+    if (c.exact)
+      k_stage2_start_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(c.X.p, c.maxr.p, M, N, 1, c.saved.p, c.chg.p);
+    else
+      k_stage2_start_w<<<cdiv(M, kRowWarps), 32 * kRowWarps, 0, c.st>>>(c.X.p, c.maxr.p, M, N);
     post_launch(c);
     if (c.exact) {
       c.xver++;  // on record: the rebuild's columns, and the placeholders' entries
@@ -2496,13 +2519,9 @@ static void outer_tail(Ctx& c, SolveState& st) {
     touch_x(c);
   } else {
     Scope s(c.timers, "doproj2");
-    const int gb = cdiv(M, 32);  // 32-row tiles
-    k_cand_proj2_t<<<dim3(gb, 1), kTileThreads, 0, c.st>>>(c.X.p, nullptr, nullptr, c.X.p, MN, c.maxr.p, M, N, 0,
-                                                         c.part2.p);
-    post_launch(c);
+    candidates_proj2(c, c.X.p, nullptr, c.X.p, 1, 0, c.sc.p + SC_TMP);
     touch_x(c);
     c.rebuilt_ver = c.xver;  // doproj2 ends with the max-column rebuild
-    reduce_to(c, c.part2.p, gb, c.sc.p + SC_TMP, 1, true, 0.0);
     read_back(c, c.sc.p + SC_TMP, 1);
     st.xmin = c.pin[0];
   }
@@ -3519,14 +3538,8 @@ int pqdts_cuda_doproj(pqdts_ctx* c) {
 int pqdts_cuda_doproj2(pqdts_ctx* c, double* xmin) {
   return guarded(c, [&] {
     pqdts::need_problem(*c);
-    const int M = (int)c->h.M, N = (int)c->h.N;
-    const int gb = pqdts::cdiv(M, 32);  // 32-row tiles
-    pqdts::k_cand_proj2_t<<<dim3(gb, 1), pqdts::kTileThreads, 0, c->st>>>(c->X.p, nullptr, nullptr, c->X.p,
-                                                                         (int64_t)M * N, c->maxr.p, M, N, 0,
-                                                                         c->part2.p);
-    pqdts::post_launch(*c);
+    pqdts::candidates_proj2(*c, c->X.p, nullptr, c->X.p, 1, 0, c->sc.p + pqdts::SC_TMP);
     pqdts::touch_x(*c);
-    pqdts::reduce_to(*c, c->part2.p, gb, c->sc.p + pqdts::SC_TMP, 1, true, 0.0);
     pqdts::read_back(*c, c->sc.p + pqdts::SC_TMP, 1);
     if (xmin) *xmin = c->pin[0];
   });
