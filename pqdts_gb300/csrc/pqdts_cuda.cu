@@ -1510,21 +1510,16 @@ static void make_map_digits(CUtensorMap* m, const void* base, uint64_t inner, ui
 
 // N tile width of a digit product over A's row blocks: the one of 64, 48,
 // 32, 16 (their six levels fit tensor memory) with the least estimated time,
-// waves of tiles x the cycles of a K chunk -- the larger of the MMAs'
-// (21 digit pairs x BN / 4 cycles a chunk) and shared memory's (128 bytes a
-// cycle: 4 KB of A per instruction, BN x 64 bytes of B per pair, twice a
-// chunk) -- so narrow tiles are taken only to fill the SMs.
+// waves of tiles x the cycles of a K chunk (21 digit pairs x BN / 2 a K slice
+// of arithmetic and ~45 of start-up for each of the 11 MMAs, two slices), so
+// narrow tiles are taken only to fill the SMs.
 static int dg_tile_n(const Ctx& c, const TcOperand& A) {
   const int N = (int)c.h.N;
   int best = 16;
-  double least = 0.0;
+  int64_t least = INT64_MAX;
   for (int bn : {64, 48, 32, 16}) {
-    int instr = 0;
-    for (int p = 0; p < kDgS; ++p) instr += cdiv((kDgS - p) * bn, 256);
-    const int pairs = kDgS * (kDgS + 1) / 2;
-    const double cyc = std::max(pairs * bn, 64 * instr + pairs * bn / 2);
-    const double t = cyc * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
-    if (least == 0.0 || t < least) {
+    const int64_t t = (int64_t)(21 * bn + 990) * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
+    if (t < least) {
       least = t;
       best = bn;
     }

@@ -24,15 +24,18 @@
 // This replaces ~12 FP32 operations a term on the CUDA cores by 21 bf16
 // MMA terms.  One CTA per SM walks a list of 128 x BN output tiles.  The
 // digits of a K chunk are one TMA box each: A 6 x 128 rows, B 6 x BN rows of
-// 64 bytes (64-byte swizzle), so with A's digit p the digits 0 .. 5 - p of B
-// are (6 - p) BN consecutive rows, and their products belong to the levels p
-// .. 5, consecutive column blocks of the accumulator: one MMA instruction
-// (or two, N <= 256) per digit of A instead of one per pair, which is what
-// keeps shared memory (A read 8 times a K slice instead of 21) below the
-// tensor pipe.  BN = 64 fills 384 of the 512 tensor-memory columns; a stage
-// is 72 KB and three fit.  The drain is not overlapped with the MMAs (no
-// room for a second accumulator), eight warps share it; the output of a
-// tile is formed and stored while the next tile's MMAs run.
+// 64 bytes (64-byte swizzle).  B's digits are stored even ones first (0 2 4 1
+// 3 5) and so are the levels' accumulators, so with one digit of A the even
+// digits of B are consecutive rows whose products belong to consecutive
+// accumulators, and the odd ones too: 11 MMA instructions a K slice, N up to
+// 192, instead of 21.  They alternate between the two halves of the
+// accumulators, for an MMA starts late behind one that it shares columns
+// with (without the alternation 9 instructions, N up to 256, took 1350
+// cycles a K slice, now ~1150, for 672 of arithmetic).  BN = 64 fills 384 of
+// the 512 tensor-memory columns; a stage is 72 KB and three fit.  The drain
+// is not overlapped with the MMAs (no room for a second accumulator), eight
+// warps share it; the output of a tile is formed, almost without the FP64
+// pipe, and stored while the next tile's MMAs run.
 #pragma once
 
 #include "tc_band.cuh"
@@ -44,6 +47,9 @@ constexpr int kDgDrain = 8;   // K chunks (of kTcK) between drains
 constexpr int kDgThreads = 320;  // TMA warp, MMA warp, 8 epilogue warps
 constexpr int kDgMaxStages = 4;
 constexpr uint32_t kDgRing = 216u * 1024u;
+
+// Place of B's digit q, and of level q's accumulator, among the six.
+__host__ __device__ constexpr int dg_slot(int q) { return (q & 1) * 3 + (q >> 1); }
 
 // Biased exponent of a double's magnitude (2047: infinite or NaN).
 __device__ __forceinline__ int dg_exponent(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff); }
@@ -90,7 +96,7 @@ __global__ void __launch_bounds__(256) k_dg_colexp(const double* __restrict__ X,
 }
 
 // Digits of X (R x N row-major) as the products' K-major operand: digit q of
-// X[r, n] at out[(q * N + n) * ld + r] (ld >= R, even).  A block transposes
+// X[r, n] at out[(dg_slot(q) * N + n) * ld + r] (ld >= R, even).  A block transposes
 // 64 rows x 32 columns through shared memory; HBM bound (8 bytes in, 12 out).
 __global__ void __launch_bounds__(256) k_dg_split_t(const double* __restrict__ X, int R, int N,
                                                     const int* __restrict__ colexp, int64_t ld,
@@ -108,7 +114,7 @@ __global__ void __launch_bounds__(256) k_dg_split_t(const double* __restrict__ X
       uint32_t d[kDgS];
       dg_digits(v, emax, d);
 #pragma unroll
-      for (int q = 0; q < kDgS; ++q) t[q][lane][y] = (uint16_t)d[q];
+      for (int q = 0; q < kDgS; ++q) t[dg_slot(q)][lane][y] = (uint16_t)d[q];
     }
   }
   __syncthreads();
@@ -175,7 +181,7 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 }
 
 // 8 consecutive columns of this thread's accumulator row in each of the six
-// levels (level stride `ls` columns), waited in place.
+// levels (ls columns each), waited in place.
 __device__ __forceinline__ void dg_ld8x6(uint32_t a, uint32_t ls, float (&v)[kDgS][8]) {
   uint32_t r[48];
   asm volatile(
@@ -192,12 +198,34 @@ __device__ __forceinline__ void dg_ld8x6(uint32_t a, uint32_t ls, float (&v)[kDg
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]),
         "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]),
         "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47])
-      : "r"(a), "r"(a + ls), "r"(a + 2 * ls), "r"(a + 3 * ls), "r"(a + 4 * ls), "r"(a + 5 * ls)
+      : "r"(a + dg_slot(0) * ls), "r"(a + dg_slot(1) * ls), "r"(a + dg_slot(2) * ls), "r"(a + dg_slot(3) * ls),
+        "r"(a + dg_slot(4) * ls), "r"(a + dg_slot(5) * ls)
       : "memory");
 #pragma unroll
   for (int q = 0; q < kDgS; ++q)
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[q][j] = __uint_as_float(r[8 * q + j]);
+}
+
+// t * 2^e as a double, rounded to nearest (halves away from zero), by the
+// integer pipes: the FP64 pipe takes 64 cycles an instruction, and a tile's
+// outputs must be formed while the next tile's first MMAs run.
+__device__ __forceinline__ double dg_value(long long t, int e) {
+  const unsigned long long u = t < 0 ? 0ull - (unsigned long long)t : (unsigned long long)t;
+  if (u == 0) return 0.0;
+  const int lz = __clzll((long long)u), be = 1023 + 63 - lz + e;  // biased exponent
+  if (be < 1 || be > 2046) return be < 1 ? 0.0 : (t < 0 ? -1.0 : 1.0) * __longlong_as_double(0x7ff0000000000000ll);
+  const unsigned long long m = u << lz;  // leading one at bit 63
+  const unsigned long long r = (m >> 11) + ((m >> 10) & 1);  // a carry raises the exponent
+  return __longlong_as_double((long long)((((unsigned long long)(be - 1) << 52) + r) |
+                                          ((unsigned long long)t & 0x8000000000000000ull)));
+}
+
+// 2 x by its bits where x is normal.
+__device__ __forceinline__ double dg_twice(double x) {
+  const long long b = __double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7ff);
+  return (unsigned)(e - 1) < 2045u ? __longlong_as_double(b + (1ll << 52)) : x + x;
 }
 
 // Operands and results of one digit product.
@@ -338,16 +366,19 @@ __global__ void __launch_bounds__(kDgThreads, 1)
               const uint32_t o = 32u * k;
 #pragma unroll
               for (int p = 0; p < kDgS; ++p) {
-                // A's digit p with B's digits 0 .. 5 - p: levels p .. 5.  The
-                // first product of a drain overwrites the accumulators: digit
-                // 0 of A does that for all levels.
+                // A's digit p with B's even digits, then its odd ones (odd p:
+                // the other way round, so that the halves of the accumulators
+                // take turns), up to digit 5 - p.  The first products of a
+                // drain overwrite the accumulators: digit 0 of A does that
+                // for all levels.
                 const uint32_t acc0 = (ch > c0 || k > 0 || p > 0) ? 1u : 0u;
-                const int cols = (kDgS - p) * BN;
                 const uint64_t da = swz_desc(sa + (uint32_t)p * a_slice + o);
-                for (int c = 0; c < cols; c += 256) {
-                  const int n = min(256, cols - c);
-                  tc_mma(tmem + (uint32_t)(p * BN + c), da, swz_desc(sb + (uint32_t)c * kTcRowBytes + o),
-                         tc_idesc_bf16(kTcRows, n), acc0);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  const int par = h ^ (p & 1), nq = (kDgS - p - par + 1) / 2;
+                  if (nq > 0)
+                    tc_mma(tmem + (uint32_t)(dg_slot(p + par) * BN), da,
+                           swz_desc(sb + (uint32_t)dg_slot(par) * b_slice + o), tc_idesc_bf16(kTcRows, nq * BN), acc0);
                 }
               }
             }
@@ -405,31 +436,54 @@ __global__ void __launch_bounds__(kDgThreads, 1)
       const int r = blk * kTcRows + q * 32 + lane;
       if (r >= g.R) continue;
       // value = acc * 2^(rowexp + colexp - 2090)
-      const int er = g.rowexp[r] - 1045;
-      const double sr = er < -1022 ? 0.0 : __longlong_as_double((long long)(er + 1023) << 52);
+      const int er = g.rowexp[r] - 2090;
       const int n0 = nt * BN + half * hc;
-      const int64_t o0 = (int64_t)r * N;
+      const int64_t o0 = (int64_t)r * N + n0;
+      // pairs of columns by 16-byte accesses where rows keep the alignment
+      const bool vec = (N & 1) == 0 && (n0 & 1) == 0;
+      const double2 zero2 = make_double2(0.0, 0.0);
 #pragma unroll
-      for (int x = 0; x < 32; ++x) {
-        const int n = n0 + x;
-        if (x >= hc || n >= N) continue;
-        const int ce = g.colexp[n], ec = ce - 1045;
-        const double sc = ec < -1022 ? 0.0 : __longlong_as_double((long long)(ec + 1023) << 52);
-        double v = (double)acc[x] * sr * sc;
-        if (ce == 2047) v = dg_plain<MODE == 4>(g, r, n);
-        const int64_t o = o0 + n;
-        if (MODE == 0) {
-          g.out[o] = 2.0 * (v - g.P[o]);
-        } else if (MODE == 3) {
-          g.out[o] = v - g.P[o];
+      for (int x = 0; x < 32; x += 2) {
+        if (x >= hc || n0 + x >= N) continue;
+        const bool two = n0 + x + 1 < N;
+        const int64_t o = o0 + x;
+        auto load = [&](const double* p) {
+          if (vec) return *reinterpret_cast<const double2*>(p);
+          return make_double2(p[0], two ? p[1] : 0.0);
+        };
+        auto store = [&](double* p, double2 y) {
+          if (vec) {
+            *reinterpret_cast<double2*>(p) = y;
+          } else {
+            p[0] = y.x;
+            if (two) p[1] = y.y;
+          }
+        };
+        const int ce0 = g.colexp[n0 + x], ce1 = two ? g.colexp[n0 + x + 1] : 0;
+        double2 v = make_double2(dg_value(acc[x], er + ce0), dg_value(acc[x + 1], er + ce1));
+        if (ce0 == 2047) v.x = dg_plain<MODE == 4>(g, r, n0 + x);
+        if (ce1 == 2047) v.y = dg_plain<MODE == 4>(g, r, n0 + x + 1);
+        if (MODE != 4) {
+          const double2 p = load(g.P + o);
+          v.x -= p.x;
+          v.y -= p.y;
+          if (MODE == 0) v = make_double2(dg_twice(v.x), dg_twice(v.y));
+          store(g.out + o, v);
         } else {
           if (g.c2gam != 0.0) {
-            const double vi = g.V[o];
-            if (r < g.R - 1) v = fma(g.c2gam, vi - g.V[o + N], v);
-            if (r > 0) v = fma(-g.c2gam, g.V[o - N] - vi, v);
+            const double2 vi = load(g.V + o);
+            const double2 vn = r < g.R - 1 ? load(g.V + o + N) : zero2, vp = r > 0 ? load(g.V + o - N) : zero2;
+            if (r < g.R - 1) {
+              v.x = fma(g.c2gam, vi.x - vn.x, v.x);
+              v.y = fma(g.c2gam, vi.y - vn.y, v.y);
+            }
+            if (r > 0) {
+              v.x = fma(-g.c2gam, vp.x - vi.x, v.x);
+              v.y = fma(-g.c2gam, vp.y - vi.y, v.y);
+            }
           }
-          if (g.out) g.out[o] = v;
-          if (g.out2) g.out2[o] = v;
+          if (g.out) store(g.out + o, v);
+          if (g.out2) store(g.out2 + o, v);
         }
       }
     }
