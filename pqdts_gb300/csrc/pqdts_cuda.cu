@@ -412,6 +412,7 @@ struct pqdts_ctx {
   // values) and, for small calls, pinned (allocated on first use)
   pqdts::DBuf<double> proj;
   double* proj_pin = nullptr;
+  double* small_pin = nullptr;  // pinned staging of small X-shaped arrays (first use)
   bool fullspace = true;
   std::vector<int32_t> h_maxr;
   pqdts::GpuTimers timers;
@@ -878,23 +879,26 @@ static void rebuild(Ctx& c, double* X, const double* saved, int32_t* chg) {
   post_launch(c);
 }
 
-// Column chains (k_colchain's OP) of B stacked inputs: a block a chain while
-// that leaves an SM at most two blocks and the chain is long enough to pay
-// for the guess (two chains of 1000 terms a column, 200 blocks: 39 us either
-// way; one: 29 against 39 by warps, 22 against 19 at 200 terms), a warp a
-// chain otherwise.
+// Column chains (k_colchain's OP) of B stacked inputs: a block a chain while that leaves
+// an SM at most two blocks and the chain is long enough to pay for the guess
+// (two chains of 1000 terms a column, 200 blocks: 39 us either way; one: 29
+// against 39 by warps), a warp a chain otherwise.  advance: the CG's scalars
+// follow (OP 2 into SC_RZ, SC_RR).
 template <int OP>
 static void launch_colchain(Ctx& c, const double* a, const double* b, int64_t stride, int B, double* out, double* out2,
-                            const double* pred, double* sum_out, int ostride, unsigned* counter) {
+                            const double* pred, double* sum_out, int ostride, unsigned* counter,
+                            bool advance = false) {
   const int M = (int)c.h.M, N = (int)c.h.N;
   const int chains = N * (OP == 2 ? 2 : 1);
+  double* sc = advance ? c.sc.p : nullptr;
   if (M >= (OP == 2 ? 1500 : 500) && (int64_t)chains * B <= (OP == 2 ? 3 : 2) * 152) {
     k_colchain_b<OP><<<dim3(chains, B), 32 * kBcWarps, 0, c.st>>>(a, b, stride, M, N, c.h.gam, out, out2, pred, sum_out,
-                                                                  ostride, counter);
+                                                                  ostride, counter, sc, c.cglog.p, kMaxCG);
   } else {
     constexpr int per = OP == 2 ? kChainWarps / 2 : kChainWarps;
     k_colchain<OP><<<dim3(cdiv(N, per), B), 32 * kChainWarps, 0, c.st>>>(a, b, stride, M, N, c.h.gam, out, out2, pred,
-                                                                         sum_out, ostride, counter);
+                                                                         sum_out, ostride, counter, sc, c.cglog.p,
+                                                                         kMaxCG);
   }
   post_launch(c);
 }
@@ -951,6 +955,10 @@ static int rows_per_block(int N) {
   return best;
 }
 
+// Whether a column product of `warps` warps has so few (at most four an SM
+// sub-partition) that each must keep its own loads ahead (col_chain_ahead).
+static bool few_warps(int64_t warps) { return warps <= 4 * 4 * 152; }
+
 // F.X (B stacked inputs, xstride apart) with the epilogue MODE of k_fwd, in
 // the context's form: column-tiled, or row-flattened (rows = 1; the same
 // bits).  cols != null: only those columns need forming (B = 1; the forms
@@ -969,9 +977,11 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
       k_col_index<T><<<dim3(cdiv(N, kIndexWarps), B), 32 * kIndexWarps, 0, c.st>>>(X, xstride, M, N, c.xcmask.p,
                                                                                   c.xccnt.p, c.xclist.p, cols);
       post_launch(c);
-      k_fwd_col<T, MODE><<<dim3(cdiv(N, kTcWarps), cdiv(D, 32), B), dim3(32, kTcWarps), 0, c.st>>>(
-          M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride, c.xcmask.p, c.xccnt.p,
-          c.xclist.p, P, R, pred, c.count_fmas ? c.fmacount.p : nullptr, cols);
+      const dim3 grid(cdiv(N, kTcWarps), cdiv(D, 32), B), block(32, kTcWarps);
+      auto kernel = few_warps((int64_t)N * grid.y * B) ? k_fwd_col<T, MODE, true> : k_fwd_col<T, MODE, false>;
+      kernel<<<grid, block, 0, c.st>>>(M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride,
+                                       c.xcmask.p, c.xccnt.p, c.xclist.p, P, R, pred,
+                                       c.count_fmas ? c.fmacount.p : nullptr, cols);
       post_launch(c);
       return;
     }
@@ -1212,9 +1222,11 @@ static void launch_trans_shape(Ctx& c, TransShape sh, const T* tv, const T* R, c
       post_launch(c);
       // with the active set (the CG's product), warps whose outputs are all
       // masked by the epilogue skip their sums
-      k_trans_col<T><<<dim3(cdiv(N, kTcWarps), cdiv(M, 32)), dim3(32, kTcWarps), 0, c.st>>>(
-          M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, acc, pred,
-          c.count_fmas ? c.fmacount.p + 1 : nullptr, ik, reduced ? c.maxr.p : nullptr, cols);
+      const dim3 grid(cdiv(N, kTcWarps), cdiv(M, 32)), block(32, kTcWarps);
+      auto kernel = few_warps((int64_t)N * grid.y) ? k_trans_col<T, true> : k_trans_col<T, false>;
+      kernel<<<grid, block, 0, c.st>>>(M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p,
+                                       c.ccnt.p, c.clist.p, acc, pred, c.count_fmas ? c.fmacount.p + 1 : nullptr, ik,
+                                       reduced ? c.maxr.p : nullptr, cols);
       post_launch(c);
       raw = acc;
     }
@@ -1335,10 +1347,10 @@ static void dot_dev(Ctx& c, const double* a, const double* b, double* out, const
 }
 
 // Two pdots of the FP64 CG at once: a.b -> out_ab, a.a -> out_aa, where
-// out_aa = out_ab + ostride (a warp per chain, two per column).
+// out_aa = out_ab + ostride; advance: then the CG's scalars.
 static void dot2_exact(Ctx& c, const double* a, const double* b, double* out_ab, int ostride,
-                       const double* pred) {
-  launch_colchain<2>(c, a, b, 0, 1, c.colbuf.p, c.colbuf.p + c.h.N, pred, out_ab, ostride, c.counters.p + 3);
+                       const double* pred, bool advance = false) {
+  launch_colchain<2>(c, a, b, 0, 1, c.colbuf.p, c.colbuf.p + c.h.N, pred, out_ab, ostride, c.counters.p + 3, advance);
 }
 
 // Hessian-vector product of one precision: Hp = H p (BF, 246-342); masks the
@@ -1870,7 +1882,7 @@ static CGGraph& captured(Ctx& c, const std::array<uint64_t, 5>& key, int spans, 
   return c.graphs.emplace(key, g).first->second;
 }
 
-// Queues CG iterations in chunks (4, then 8) and polls the exit flag after
+// Queues CG iterations in chunks of 4 and polls the exit flag after
 // each chunk; iterations queued after the exit are no-ops (each kernel reads
 // the flag first), the flag is also set at the iteration limit.  With graphs
 // on, a chunk is one replay of a captured graph.  Returns the iterations run.
@@ -1879,7 +1891,7 @@ static int cg_chunks(Ctx& c, std::array<uint64_t, 4> variant, Iter&& iteration) 
   int queued = 0;
   for (int chunk_no = 0;; ++chunk_no) {
     const bool first = chunk_no == 0;
-    const int chunk = first ? 4 : 8;
+    const int chunk = 4;
     if (c.use_graphs) {
       const int spans = chunk * (c.timers.detail ? 8 : 1);  // timer spans recorded per chunk
       CGGraph& gr = captured(c, {variant[0], variant[1], variant[2], variant[3], (uint64_t)first}, spans, [&] {
@@ -2058,14 +2070,14 @@ static void cg_solve(Ctx& c, CGBufs<T>& b, const T* fv, const T* tv, double bdfa
     if (exact) {
       if constexpr (kF64) {
         static_assert(SC_RR - SC_RZ == 1, "scalar layout");
-        dot2_exact(c, b.r.p, b.z.p, c.sc.p + SC_RZ, 1, c.sc.p);
+        dot2_exact(c, b.r.p, b.z.p, c.sc.p + SC_RZ, 1, c.sc.p, true);
       }
     } else {
       reduce_to(c, c.part.p, g, c.sc.p + SC_RZ, 1, false, 0.0, c.sc.p);
       reduce_to(c, c.part2.p, g, c.sc.p + SC_RR, 1, false, 0.0, c.sc.p);
+      k_cg_scalars1<<<1, 1, 0, c.st>>>(c.sc.p, c.cglog.p, kMaxCG);
+      post_launch(c);
     }
-    k_cg_scalars1<<<1, 1, 0, c.st>>>(c.sc.p, c.cglog.p, kMaxCG);
-    post_launch(c);
   };
   uint64_t bdbits;
   std::memcpy(&bdbits, &bdfac, 8);
@@ -2569,22 +2581,52 @@ static void run_stage(Ctx& c, int mode, int oiter, int maxiiter, double conv_thr
 // staging copy is entry `slot` of the line-search candidates' stack, whose
 // contents outlive a line search only up to the update that adopts one of
 // them (outer_tail), never an entry point.
+//
+// Up to kHostTranspose entries the host turns the array round itself, in
+// pinned memory (slots 0 and 1 for what goes up, 2 for what comes down): a
+// launch and its latency, ~5 us an array, cost more than such a loop (BF32 at
+// M = 280, N = 27: 83 us with both arrays turned round on the device).
+constexpr int64_t kHostTranspose = 8192;
+
+template <typename T>
+static T* small_stage(Ctx& c, int slot) {
+  if (!c.small_pin) CK(cudaMallocHost((void**)&c.small_pin, 3 * kHostTranspose * sizeof(double)));
+  return reinterpret_cast<T*>(c.small_pin + slot * kHostTranspose);
+}
+
 template <typename T>
 static void upload_colmajor(Ctx& c, const double* in, T* dev, int slot = 0) {
   const int M = (int)c.h.M, N = (int)c.h.N;
   const int64_t MN = (int64_t)M * N;
+  if (MN <= kHostTranspose) {
+    T* rm = small_stage<T>(c, slot);
+    for (int i = 0; i < M; ++i)
+      for (int n = 0; n < N; ++n) rm[(size_t)i * N + n] = (T)in[i + (int64_t)n * M];
+    CK(cudaMemcpyAsync(dev, rm, MN * sizeof(T), cudaMemcpyHostToDevice, c.st));
+    return;
+  }
   double* stage = c.Xc.p + slot * MN;
   CK(cudaMemcpyAsync(stage, in, MN * sizeof(double), cudaMemcpyHostToDevice, c.st));
   k_transpose<double, T><<<cdiv(M, 32) * cdiv(N, 32), 256, 0, c.st>>>(stage, N, M, dev);
   post_launch(c);
 }
 
+// (waits for the stream)
 template <typename T>
 static void download_colmajor(Ctx& c, const T* dev, double* out) {
   const int M = (int)c.h.M, N = (int)c.h.N;
+  const int64_t MN = (int64_t)M * N;
+  if (MN <= kHostTranspose) {
+    T* rm = small_stage<T>(c, 2);
+    CK(cudaMemcpyAsync(rm, dev, MN * sizeof(T), cudaMemcpyDeviceToHost, c.st));
+    CK(cudaStreamSynchronize(c.st));
+    for (int i = 0; i < M; ++i)
+      for (int n = 0; n < N; ++n) out[i + (int64_t)n * M] = (double)rm[(size_t)i * N + n];
+    return;
+  }
   k_transpose<T, double><<<cdiv(M, 32) * cdiv(N, 32), 256, 0, c.st>>>(dev, M, N, c.Xc.p);
   post_launch(c);
-  CK(cudaMemcpyAsync(out, c.Xc.p, (int64_t)M * N * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  CK(cudaMemcpyAsync(out, c.Xc.p, MN * sizeof(double), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
 }
 
@@ -3287,6 +3329,7 @@ int pqdts_cuda_destroy(pqdts_ctx* c) {
   if (c->st) cudaStreamSynchronize(c->st);
   if (c->pin) cudaFreeHost(c->pin);
   if (c->proj_pin) cudaFreeHost(c->proj_pin);
+  if (c->small_pin) cudaFreeHost(c->small_pin);
   cudaStream_t st = c->own_stream ? c->st : nullptr;
   delete c;
   if (st) cudaStreamDestroy(st);
@@ -3492,9 +3535,9 @@ int pqdts_cuda_BF32(pqdts_ctx* c, const double* V, double* HV) {
       pqdts::post_launch(*c);
     }
     pqdts::hvp32(*c, b, nullptr, false, nullptr);
-    pqdts::read_back(*c, c->sc.p, pqdts::SC_NSC);
-    pqdts::check_tc_error(*c);
+    CK(cudaMemcpyAsync(c->pin, c->sc.p, pqdts::SC_NSC * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     pqdts::download_colmajor(*c, b.Hp.p, HV);
+    pqdts::check_tc_error(*c);
     c->d2h += M * N * 8;
   });
 }
