@@ -956,7 +956,7 @@ static int rows_per_block(int N) {
 }
 
 // Whether a column product of `warps` warps has so few (at most four an SM
-// sub-partition) that each must keep its own loads ahead (col_chain_ahead).
+// sub-partition) that each is better fed by another (fed_chain).
 static bool few_warps(int64_t warps) { return warps <= 4 * 4 * 152; }
 
 // F.X (B stacked inputs, xstride apart) with the epilogue MODE of k_fwd, in
@@ -977,11 +977,16 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
       k_col_index<T><<<dim3(cdiv(N, kIndexWarps), B), 32 * kIndexWarps, 0, c.st>>>(X, xstride, M, N, c.xcmask.p,
                                                                                   c.xccnt.p, c.xclist.p, cols);
       post_launch(c);
-      const dim3 grid(cdiv(N, kTcWarps), cdiv(D, 32), B), block(32, kTcWarps);
-      auto kernel = few_warps((int64_t)N * grid.y * B) ? k_fwd_col<T, MODE, true> : k_fwd_col<T, MODE, false>;
-      kernel<<<grid, block, 0, c.st>>>(M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride,
-                                       c.xcmask.p, c.xccnt.p, c.xclist.p, P, R, pred,
-                                       c.count_fmas ? c.fmacount.p : nullptr, cols);
+      const int tiles = cdiv(D, 32);
+      unsigned long long* count = c.count_fmas ? c.fmacount.p : nullptr;
+      if (few_warps((int64_t)N * tiles * B))
+        k_fwd_fed<MODE><<<dim3(cdiv(N, 2), tiles, B), dim3(32, 4), 0, c.st>>>(
+            M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride, c.xcmask.p, c.xccnt.p,
+            c.xclist.p, P, R, pred, count, cols);
+      else
+        k_fwd_col<T, MODE><<<dim3(cdiv(N, kTcWarps), tiles, B), dim3(32, kTcWarps), 0, c.st>>>(
+            M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride, c.xcmask.p, c.xccnt.p,
+            c.xclist.p, P, R, pred, count, cols);
       post_launch(c);
       return;
     }
@@ -1222,11 +1227,16 @@ static void launch_trans_shape(Ctx& c, TransShape sh, const T* tv, const T* R, c
       post_launch(c);
       // with the active set (the CG's product), warps whose outputs are all
       // masked by the epilogue skip their sums
-      const dim3 grid(cdiv(N, kTcWarps), cdiv(M, 32)), block(32, kTcWarps);
-      auto kernel = few_warps((int64_t)N * grid.y) ? k_trans_col<T, true> : k_trans_col<T, false>;
-      kernel<<<grid, block, 0, c.st>>>(M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p,
-                                       c.ccnt.p, c.clist.p, acc, pred, c.count_fmas ? c.fmacount.p + 1 : nullptr, ik,
-                                       reduced ? c.maxr.p : nullptr, cols);
+      const int tiles = cdiv(M, 32);
+      unsigned long long* count = c.count_fmas ? c.fmacount.p + 1 : nullptr;
+      if (few_warps((int64_t)N * tiles))
+        k_trans_fed<<<dim3(cdiv(N, 2), tiles), dim3(32, 4), 0, c.st>>>(
+            M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, acc, pred,
+            count, ik, reduced ? c.maxr.p : nullptr, cols);
+      else
+        k_trans_col<T><<<dim3(cdiv(N, kTcWarps), tiles), dim3(32, kTcWarps), 0, c.st>>>(
+            M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, acc, pred,
+            count, ik, reduced ? c.maxr.p : nullptr, cols);
       post_launch(c);
       raw = acc;
     }
