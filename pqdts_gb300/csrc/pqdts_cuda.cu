@@ -707,9 +707,11 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
     c.df_trans = c.df_fwd && c.t_contiguous;
     CK(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
     // by digits on the tensor cores unless double-FP32 (df_products = 1) or
-    // CUDA cores (tensor_cores = 0) are asked for; a digit needs a finite F
-    c.dg_fwd = c.df_option < 0 && c.f_finite && tc_wanted(c);
-    c.dg_trans = c.dg_fwd && c.t_contiguous;
+    // CUDA cores (tensor_cores = 0) are asked for; a digit needs a finite F,
+    // and the sums that they are collected in hold so many terms
+    const auto widest = [](const std::vector<int32_t>& w) { return w.empty() ? 0 : *std::max_element(w.begin(), w.end()); };
+    c.dg_fwd = c.df_option < 0 && c.f_finite && widest(h.fw) < kDgMaxFwd && tc_wanted(c);
+    c.dg_trans = c.dg_fwd && c.t_contiguous && widest(h.tw) < kDgMaxTrans;
     if (c.df_fwd && !c.dg_fwd) {
       c.fdf.alloc(nnz);
       k_split_df<<<elem_grid(nnz), 256, 0, c.st>>>(c.fval.p, nnz, 1.0, c.fdf.p);
@@ -1004,6 +1006,7 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
 
 // The mixed path's digit products read `rows` x N doubles of B as digits of
 // each column's scale: the columns' exponents, then the transposed digits.
+template <int S>
 static void dg_split(Ctx& c, const double* B, int rows, int64_t ld, DBuf<uint16_t>& dig) {
   const int N = (int)c.h.N;
   CK(cudaMemsetAsync(c.dg_colexp.p, 0, N * sizeof(int), c.st));
@@ -1011,7 +1014,7 @@ static void dg_split(Ctx& c, const double* B, int rows, int64_t ld, DBuf<uint16_
   const int shares = std::max(1, std::min(cdiv(rows, 64), cdiv((int64_t)4 * c.num_sms, cdiv(N, 32))));
   k_dg_colexp<<<dim3(cdiv(N, 32), shares), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p);
   post_launch(c);
-  k_dg_split_t<<<dim3(cdiv(rows, 64), cdiv(N, 32)), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p, ld, dig.p);
+  k_dg_split_t<S><<<dim3(cdiv(rows, 64), cdiv(N, 32)), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p, ld, dig.p);
   post_launch(c);
 }
 
@@ -1052,7 +1055,7 @@ template <int MODE>
 static void fwd_df(Ctx& c, const double* X, double* R) {
   const int64_t MN = c.h.M * c.h.N;
   if (c.dg_fwd) {
-    dg_split(c, X, (int)c.h.M, c.tc_mp, c.dg_x);
+    dg_split<kDgFwd>(c, X, (int)c.h.M, c.tc_mp, c.dg_x);
     dg_product<MODE>(c, c.dgF, c.tcF, (int)c.h.D, X, R, nullptr, nullptr, 0.0);
     return;
   }
@@ -1304,7 +1307,7 @@ static void op_dL(Ctx& c) {
     double* g = c.fullspace ? c.G.p : nullptr;
     const double c2g = 2.0 * c.h.gam;
     if (c.dg_trans) {
-      dg_split(c, c.R.p, D, c.tc_dp, c.dg_r);
+      dg_split<kDgTrans>(c, c.R.p, D, c.tc_dp, c.dg_r);
       dg_product<4>(c, c.dgFt, c.tcFt, M, c.R.p, c.Gf.p, g, c.X.p, c2g);
     } else {
       k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p);
@@ -1515,13 +1518,13 @@ static void setup_tc(Ctx& c) {
   c.tc_ready = true;
 }
 
-// 3-D bf16 map of an operand's digits: inner x rows x kDgS, box kTcK x
-// box_rows x kDgS, swizzled to the stage's row width, zero fill outside.
+// 3-D bf16 map of an operand's digits: inner x rows x digits, box kTcK x
+// box_rows x digits, swizzled to the stage's row width, zero fill outside.
 static void make_map_digits(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint64_t row_elems,
-                            uint32_t box_rows) {
-  const cuuint64_t dims[3] = {inner, rows, (cuuint64_t)kDgS};
+                            uint32_t box_rows, int digits) {
+  const cuuint64_t dims[3] = {inner, rows, (cuuint64_t)digits};
   const cuuint64_t strides[2] = {row_elems * 2, rows * row_elems * 2};
-  const cuuint32_t box[3] = {(cuuint32_t)kTcK, box_rows, (cuuint32_t)kDgS};
+  const cuuint32_t box[3] = {(cuuint32_t)kTcK, box_rows, (cuuint32_t)digits};
   const cuuint32_t es[3] = {1, 1, 1};
   static_assert(kTcRowBytes == 64, "the swizzle below");
   const CUresult r = encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box,
@@ -1531,16 +1534,16 @@ static void make_map_digits(CUtensorMap* m, const void* base, uint64_t inner, ui
 }
 
 // N tile width of a digit product over A's row blocks: the one of 64, 48,
-// 32, 16 (their six levels fit tensor memory) with the least estimated time,
-// waves of tiles x the cycles of a K chunk (21 digit pairs x BN / 2 a K slice
-// of arithmetic and ~45 of start-up for each of the 11 MMAs, two slices), so
-// narrow tiles are taken only to fill the SMs.
-static int dg_tile_n(const Ctx& c, const TcOperand& A) {
+// 32, 16 (their six or seven levels fit tensor memory) with the least estimated
+// time, waves of tiles x the cycles of a K chunk (21 or 28 digit pairs x BN / 2
+// a K slice of arithmetic and ~45 of start-up for each of the 11 MMAs, two
+// slices), so narrow tiles are taken only to fill the SMs.
+static int dg_tile_n(const Ctx& c, const TcOperand& A, int digits) {
   const int N = (int)c.h.N;
   int best = 16;
   int64_t least = INT64_MAX;
   for (int bn : {64, 48, 32, 16}) {
-    const int64_t t = (int64_t)(21 * bn + 990) * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
+    const int64_t t = (int64_t)(digits * (digits + 1) / 2 * bn + 990) * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
     if (t < least) {
       least = t;
       best = bn;
@@ -1554,19 +1557,20 @@ static int dg_tile_n(const Ctx& c, const TcOperand& A) {
 static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf<uint16_t>& dig_b, int64_t K,
                          int64_t ld) {
   const int N = (int)c.h.N, rows = win.blocks * kTcRows;
-  op.dig.alloc((size_t)kDgS * rows * win.kmax);
+  const int S = trans ? kDgTrans : kDgFwd;
+  op.dig.alloc((size_t)S * rows * win.kmax);
   op.rowexp.alloc(rows);
-  dig_b.alloc((size_t)kDgS * N * ld);
+  dig_b.alloc((size_t)S * N * ld);
   if (trans)
     k_dg_band<true><<<rows, 256, 0, c.st>>>(bands_of(c), c.tval.p, win.kb.p, rows, win.kmax, op.dig.p, op.rowexp.p);
   else
     k_dg_band<false><<<rows, 256, 0, c.st>>>(bands_of(c), c.fval.p, win.kb.p, rows, win.kmax, op.dig.p, op.rowexp.p);
   post_launch(c);
-  op.bn = dg_tile_n(c, win);
-  const uint32_t stage = kDgS * (kTcRows + (uint32_t)op.bn) * kTcRowBytes;
+  op.bn = dg_tile_n(c, win, S);
+  const uint32_t stage = S * (kTcRows + (uint32_t)op.bn) * kTcRowBytes;
   op.stages = std::min<int>(kDgMaxStages, (int)(kDgRing / stage));
-  make_map_digits(&op.map_a, op.dig.p, win.kmax, rows, win.kmax, kTcRows);
-  make_map_digits(&op.map_b, dig_b.p, K, N, ld, (uint32_t)op.bn);
+  make_map_digits(&op.map_a, op.dig.p, win.kmax, rows, win.kmax, kTcRows, S);
+  make_map_digits(&op.map_b, dig_b.p, K, N, ld, (uint32_t)op.bn, S);
   // tiles from the last row block down (the widest K windows of a Poisson F
   // first), each to the CTA with the least work so far: the CTAs stay within
   // a few row blocks of one another, so A's digits are read from HBM once
@@ -1596,9 +1600,8 @@ static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf
 static void setup_dg(Ctx& c) {
   if (!c.dg_fwd) return;
   c.dg_colexp.alloc(c.h.N);
-  CK(cudaFuncSetAttribute(k_dg_band_product<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
-  CK(cudaFuncSetAttribute(k_dg_band_product<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
-  CK(cudaFuncSetAttribute(k_dg_band_product<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
+  for (auto k : {k_dg_band_product<0>, k_dg_band_product<3>, k_dg_band_product<4>})
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
   setup_digits(c, c.dgF, c.tcF, false, c.dg_x, c.h.M, c.tc_mp);
   if (c.dg_trans) setup_digits(c, c.dgFt, c.tcFt, true, c.dg_r, c.h.D, c.tc_dp);
 }

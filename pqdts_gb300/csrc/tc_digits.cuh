@@ -4,9 +4,8 @@
 //
 // Every operand row of F (or F^T) and every column of X (or R) is scaled by
 // a power of two, so that its largest magnitude lies in [1/4, 1/2), rounded
-// to 48 bits and written as kDgS = 6 signed digits in base 256, each exact
-// in bf16:
-//   x = 2^E (d_0 2^-8 + d_1 2^-16 + ... + d_5 2^-48),  |d_q| <= 128.
+// to 8 S bits and written as S signed digits in base 256, each exact in bf16:
+//   x = 2^E (d_0 2^-8 + d_1 2^-16 + ... ),  |d_q| <= 128.
 // A product is then a sum over digit pairs, and the pairs p + q = L of one
 // level L share a weight 2^(-8 (L + 2)), so level L needs one integer sum
 //   S_L = sum_k sum_{p + q = L} dF_p[k] dX_q[k]
@@ -14,62 +13,78 @@
 // a product of digits is at most 2^14, and the accumulators are drained into
 // 64-bit integers every kDgDrain = 8 chunks of K = 32, so a pair's sum stays
 // within 256 * 2^14 = 2^22 and the levels 0..3 within 2^24, the integers an
-// FP32 accumulator holds; levels 4 and 5 may pass that (by at most 1.5x,
-// operands whose digits all have one sign) and then round by an ulp, 2^-48
-// of the scales.  Levels 0..5 are kept (21 digit pairs): the error of a sum
-// is ~sqrt(K) 2^-47 of (row scale x column scale), measured against 64 bits
-// 2e-15 to 6e-15 of the result's norm where the double-FP32 kernels
-// (k_fwd_df, k_trans_df) are 1.3e-14 to 4e-14 off.
+// FP32 accumulator holds; the next ones may pass that (by at most 1.75x,
+// operands whose digits all have one sign) and then round by an ulp.  The
+// levels 0 .. S - 1 are kept, S (S + 1) / 2 digit pairs: the error of a sum
+// is ~sqrt(K) 2^(1 - 8 S) of (row scale x column scale).
 //
-// This replaces ~12 FP32 operations a term on the CUDA cores by 21 bf16
-// MMA terms.  One CTA per SM walks a list of 128 x BN output tiles.  The
-// digits of a K chunk are one TMA box each: A 6 x 128 rows, B 6 x BN rows of
-// 64 bytes (64-byte swizzle).  B's digits are stored even ones first (0 2 4 1
-// 3 5) and so are the levels' accumulators, so with one digit of A the even
+// S = 6 for F^T.R.  S = 7 for F.X, whose difference from P cancels and leaves
+// that error larger beside it: at iterates with most entries zero six digits
+// left the gradient 1.0-1.7 times (M = 200-400), 0.7 (M = 900), 0.2 times (M =
+// 4000-10^4, single entries up to 1.6 times) as far from 64-bit arithmetic as
+// the double-FP32 kernels (k_fwd_df, k_trans_df) do, seven 0.07-0.4 times at
+// M = 200-400 and 0.04-0.1 above (dense iterates: 0.04-0.25), for 2 % more
+// time of F.X at M = 6000 and 11 % at M = 10^4.
+//
+// This replaces ~12 FP32 operations a term on the CUDA cores by 28 (F^T: 21)
+// bf16 MMA terms.  One CTA per SM walks a list of 128 x BN output tiles.  The
+// digits of a K chunk are one TMA box each: A S x 128 rows, B S x BN rows of
+// 64 bytes (64-byte swizzle).  B's digits are stored even ones first (0 2 4 6
+// 1 3 5) and so are the levels' accumulators, so with one digit of A the even
 // digits of B are consecutive rows whose products belong to consecutive
-// accumulators, and the odd ones too: 11 MMA instructions a K slice, N up to
-// 192, instead of 21.  They alternate between the two halves of the
-// accumulators, for an MMA starts late behind one that it shares columns
-// with (without the alternation 9 instructions, N up to 256, took 1350
-// cycles a K slice, now ~1150, for 672 of arithmetic).  BN = 64 fills 384 of
-// the 512 tensor-memory columns; a stage is 72 KB and three fit.  The drain
-// is not overlapped with the MMAs (no room for a second accumulator), eight
-// warps share it; the output of a tile is formed, almost without the FP64
-// pipe, and stored while the next tile's MMAs run.
+// accumulators, and the odd ones too: 13 (11) MMA instructions a K slice, N up
+// to 256 (192), instead of 28 (21).  They alternate between the two halves of
+// the accumulators, for an MMA starts late behind one that it shares columns
+// with (S = 6: without the alternation 9 instructions, N up to 256, took 1350
+// cycles a K slice, now ~1150, for 672 of arithmetic).  BN = 64 fills 448
+// (384) of the 512 tensor-memory columns; a stage is 84 (72) KB and two
+// (three) fit.  The drain is not overlapped with the MMAs (no room for a
+// second accumulator), eight warps share it; the output of a tile is formed,
+// almost without the FP64 pipe, and stored while the next tile's MMAs run.
 #pragma once
 
 #include "tc_band.cuh"
 
 namespace pqdts {
 
-constexpr int kDgS = 6;       // base-256 digits an operand
+constexpr int kDgFwd = 7, kDgTrans = 6;  // base-256 digits an operand
+// The sums, in units of 2^-52 (2^-48) of the scales, stay below 2^63 for so
+// many terms of at most 1/2 x 1/2.
+constexpr int kDgMaxFwd = 1 << 13, kDgMaxTrans = 1 << 17;
 constexpr int kDgDrain = 8;   // K chunks (of kTcK) between drains
 constexpr int kDgThreads = 320;  // TMA warp, MMA warp, 8 epilogue warps
 constexpr int kDgMaxStages = 4;
 constexpr uint32_t kDgRing = 216u * 1024u;
 
-// Place of B's digit q, and of level q's accumulator, among the six.
-__host__ __device__ constexpr int dg_slot(int q) { return (q & 1) * 3 + (q >> 1); }
+// Place of B's digit q, and of level q's accumulator, among S.
+template <int S>
+__host__ __device__ constexpr int dg_slot(int q) {
+  return (q & 1) * ((S + 1) / 2) + (q >> 1);
+}
 
 // Biased exponent of a double's magnitude (2047: infinite or NaN).
 __device__ __forceinline__ int dg_exponent(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff); }
 
-// The kDgS digits (bf16 bit patterns, most significant first) of v, whose
-// biased exponent is at most emax: v = 2^(emax - 1069) t, t = v's mantissa
-// shifted to the scale's 48 bits, rounded half away from zero; each byte of
-// t + 0x808080808080 is a digit + 128.
-__device__ __forceinline__ void dg_digits(double v, int emax, uint32_t (&d)[kDgS]) {
+// The S digits (bf16 bit patterns, most significant first) of v, whose biased
+// exponent is at most emax: v = 2^(emax - 1021 - 8 S) t, t = v's mantissa
+// shifted to the scale's 8 S bits, rounded half away from zero; each byte of
+// t + 0x8080...80 is a digit + 128.
+template <int S>
+__device__ __forceinline__ void dg_digits(double v, int emax, uint32_t (&d)[S]) {
   const long long b = __double_as_longlong(v);
   int e = (int)((b >> 52) & 0x7ff);
   unsigned long long m = (unsigned long long)b & ((1ull << 52) - 1);
   if (e != 0) m |= 1ull << 52;
   else e = 1;
-  const int sh = max(emax, 1) - e + 6;  // >= 6
-  const unsigned long long t = sh <= 54 ? (m + (1ull << (sh - 1))) >> sh : 0ull;  // <= 2^47
-  const unsigned long long u = (b < 0 ? 0ull - t : t) + 0x808080808080ull;
+  const int sh = max(emax, 1) - e + 54 - 8 * S;  // >= 54 - 8 S
+  unsigned long long t;  // <= 2^(8 S - 1)
+  if (S == 7 && sh <= 0) t = m << -sh;
+  else t = sh <= 54 ? (m + (1ull << (sh - 1))) >> sh : 0ull;
+  constexpr unsigned long long bias = 0x8080808080808080ull >> (64 - 8 * S);
+  const unsigned long long u = (b < 0 ? 0ull - t : t) + bias;
 #pragma unroll
-  for (int q = 0; q < kDgS; ++q) {
-    const uint32_t byte = (uint32_t)(u >> (8 * (kDgS - 1 - q))) & (q == 0 ? 0x1ffu : 0xffu);
+  for (int q = 0; q < S; ++q) {
+    const uint32_t byte = (uint32_t)(u >> (8 * (S - 1 - q))) & (q == 0 ? 0x1ffu : 0xffu);
     // 2^23 + byte as a float, minus 2^23 + 128: the digit, exactly
     d[q] = __float_as_uint(__fsub_rn(__uint_as_float(0x4b000000u | byte), 8388736.0f)) >> 16;
   }
@@ -96,12 +111,13 @@ __global__ void __launch_bounds__(256) k_dg_colexp(const double* __restrict__ X,
 }
 
 // Digits of X (R x N row-major) as the products' K-major operand: digit q of
-// X[r, n] at out[(dg_slot(q) * N + n) * ld + r] (ld >= R, even).  A block transposes
+// X[r, n] at out[(dg_slot<S>(q) * N + n) * ld + r] (ld >= R, even).  A block transposes
 // 64 rows x 32 columns through shared memory; HBM bound (8 bytes in, 12 out).
+template <int S>
 __global__ void __launch_bounds__(256) k_dg_split_t(const double* __restrict__ X, int R, int N,
                                                     const int* __restrict__ colexp, int64_t ld,
                                                     uint16_t* __restrict__ out) {
-  __shared__ __align__(4) uint16_t t[kDgS][32][66];
+  __shared__ __align__(4) uint16_t t[S][32][66];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int r0 = blockIdx.x * 64, n0 = blockIdx.y * 32;
   {
@@ -111,16 +127,16 @@ __global__ void __launch_bounds__(256) k_dg_split_t(const double* __restrict__ X
     for (int k = 0; k < 8; ++k) {
       const int y = w + 8 * k, r = r0 + y;
       const double v = (r < R && n < N) ? X[(int64_t)r * N + n] : 0.0;
-      uint32_t d[kDgS];
-      dg_digits(v, emax, d);
+      uint32_t d[S];
+      dg_digits<S>(v, emax, d);
 #pragma unroll
-      for (int q = 0; q < kDgS; ++q) t[dg_slot(q)][lane][y] = (uint16_t)d[q];
+      for (int q = 0; q < S; ++q) t[dg_slot<S>(q)][lane][y] = (uint16_t)d[q];
     }
   }
   __syncthreads();
   const int r = r0 + 2 * lane;
 #pragma unroll 4
-  for (int x = w; x < kDgS * 32; x += 8) {
+  for (int x = w; x < S * 32; x += 8) {
     const int q = x >> 5, n = n0 + (x & 31);
     if (n >= N || r >= R) continue;
     uint16_t* o = out + ((int64_t)q * N + n) * ld + r;
@@ -137,6 +153,7 @@ template <bool TRANS>
 __global__ void __launch_bounds__(256) k_dg_band(DevBands f, const double* __restrict__ val,
                                                  const int32_t* __restrict__ kb, int rows, int kmax,
                                                  uint16_t* __restrict__ out, int* __restrict__ rowexp) {
+  constexpr int S = TRANS ? kDgTrans : kDgFwd;
   __shared__ int s_e;
   const int r = blockIdx.x, R = TRANS ? f.M : f.D;
   int lo = 0, w = 0;
@@ -164,10 +181,10 @@ __global__ void __launch_bounds__(256) k_dg_band(DevBands f, const double* __res
   for (int x = threadIdx.x; x < kmax; x += blockDim.x) {
     const int k = x - start;
     const double v = (unsigned)k < (unsigned)w ? val[off + k] : 0.0;
-    uint32_t d[kDgS];
-    dg_digits(v, e, d);
+    uint32_t d[S];
+    dg_digits<S>(v, e, d);
 #pragma unroll
-    for (int q = 0; q < kDgS; ++q) out[((int64_t)q * rows + r) * kmax + x] = (uint16_t)d[q];
+    for (int q = 0; q < S; ++q) out[((int64_t)q * rows + r) * kmax + x] = (uint16_t)d[q];
   }
 }
 
@@ -180,9 +197,10 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-// 8 consecutive columns of this thread's accumulator row in each of the six
+// 8 consecutive columns of this thread's accumulator row in each of the S
 // levels (ls columns each), waited in place.
-__device__ __forceinline__ void dg_ld8x6(uint32_t a, uint32_t ls, float (&v)[kDgS][8]) {
+template <int S>
+__device__ __forceinline__ void dg_ld8(uint32_t a, uint32_t ls, float (&v)[S][8]) {
   uint32_t r[48];
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%48];\n\t"
@@ -198,13 +216,23 @@ __device__ __forceinline__ void dg_ld8x6(uint32_t a, uint32_t ls, float (&v)[kDg
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]),
         "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]),
         "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47])
-      : "r"(a + dg_slot(0) * ls), "r"(a + dg_slot(1) * ls), "r"(a + dg_slot(2) * ls), "r"(a + dg_slot(3) * ls),
-        "r"(a + dg_slot(4) * ls), "r"(a + dg_slot(5) * ls)
+      : "r"(a + dg_slot<S>(0) * ls), "r"(a + dg_slot<S>(1) * ls), "r"(a + dg_slot<S>(2) * ls),
+        "r"(a + dg_slot<S>(3) * ls), "r"(a + dg_slot<S>(4) * ls), "r"(a + dg_slot<S>(5) * ls)
       : "memory");
 #pragma unroll
-  for (int q = 0; q < kDgS; ++q)
+  for (int q = 0; q < 6; ++q)
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[q][j] = __uint_as_float(r[8 * q + j]);
+  if constexpr (S == 7) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(a + dg_slot<S>(6) * ls)
+        : "memory");
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[S - 1][j] = __uint_as_float(r[j]);
+  }
 }
 
 // t * 2^e as a double, rounded to nearest (halves away from zero), by the
@@ -275,6 +303,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kDgThreads, 1)
     k_dg_band_product(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
                       const __grid_constant__ DgArgs g) {
+  constexpr int S = MODE == 4 ? kDgTrans : kDgFwd;
   extern __shared__ uint8_t tc_smem_raw[];
   __shared__ uint64_t bar_full[kDgMaxStages], bar_empty[kDgMaxStages], bar_accf, bar_acce, bar_fin;
   __shared__ uint32_t s_tmem;
@@ -287,8 +316,8 @@ __global__ void __launch_bounds__(kDgThreads, 1)
   const uint32_t raw = smem_u32(tc_smem_raw);
   uint8_t* base = tc_smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   const uint32_t a_slice = kTcRows * kTcRowBytes, b_slice = (uint32_t)BN * kTcRowBytes;
-  const uint32_t a_bytes = kDgS * a_slice, stage_bytes = a_bytes + kDgS * b_slice;
-  const uint32_t ncols = kDgS * BN <= 128 ? 128u : kDgS * BN <= 256 ? 256u : 512u;
+  const uint32_t a_bytes = S * a_slice, stage_bytes = a_bytes + S * b_slice;
+  const uint32_t ncols = S * BN <= 128 ? 128u : S * BN <= 256 ? 256u : 512u;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&mA);
@@ -365,20 +394,21 @@ __global__ void __launch_bounds__(kDgThreads, 1)
             for (int k = 0; k < kTcK / 16; ++k) {
               const uint32_t o = 32u * k;
 #pragma unroll
-              for (int p = 0; p < kDgS; ++p) {
+              for (int p = 0; p < S; ++p) {
                 // A's digit p with B's even digits, then its odd ones (odd p:
                 // the other way round, so that the halves of the accumulators
-                // take turns), up to digit 5 - p.  The first products of a
+                // take turns), up to digit S - 1 - p.  The first products of a
                 // drain overwrite the accumulators: digit 0 of A does that
                 // for all levels.
                 const uint32_t acc0 = (ch > c0 || k > 0 || p > 0) ? 1u : 0u;
                 const uint64_t da = swz_desc(sa + (uint32_t)p * a_slice + o);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                  const int par = h ^ (p & 1), nq = (kDgS - p - par + 1) / 2;
+                  const int par = h ^ (p & 1), nq = (S - p - par + 1) / 2;
                   if (nq > 0)
-                    tc_mma(tmem + (uint32_t)(dg_slot(p + par) * BN), da,
-                           swz_desc(sb + (uint32_t)dg_slot(par) * b_slice + o), tc_idesc_bf16(kTcRows, nq * BN), acc0);
+                    tc_mma(tmem + (uint32_t)(dg_slot<S>(p + par) * BN), da,
+                           swz_desc(sb + (uint32_t)dg_slot<S>(par) * b_slice + o), tc_idesc_bf16(kTcRows, nq * BN),
+                           acc0);
                 }
               }
             }
@@ -399,8 +429,9 @@ __global__ void __launch_bounds__(kDgThreads, 1)
     for (int j = j_begin; j < j_end && ok; ++j) {
       const int t = g.sched_tile[j], nt = t % ntn, blk = t / ntn;
       const int nk = g.kb[blk] >= 0 ? g.nch[blk] : 0;
-      // sums in units of 2^48 of the digits' least product weight (level 4);
-      // level 5 enters rounded to it
+      // sums in units of level 4's weight (S = 7: a sixteenth of it); the
+      // levels below enter rounded to the unit
+      constexpr int fine = S == 7 ? 4 : 0;
       long long acc[32];
 #pragma unroll
       for (int x = 0; x < 32; ++x) acc[x] = 0;
@@ -413,17 +444,20 @@ __global__ void __launch_bounds__(kDgThreads, 1)
 #pragma unroll
         for (int x = 0; x < 32; x += 8)
           if (x < hc) {
-            float v[kDgS][8];
-            dg_ld8x6(ta + (uint32_t)x, (uint32_t)BN, v);
+            float v[S][8];
+            dg_ld8<S>(ta + (uint32_t)x, (uint32_t)BN, v);
 #pragma unroll
             for (int y = 0; y < 8; ++y) {
-              const int l4 = __float2int_rn(fmaf(v[5][y], 0.00390625f, v[4][y]));
-              long long s = acc[x + y] + l4;
-              s += (long long)__float2int_rn(v[3][y]) * 256;
-              s += (long long)__float2int_rn(v[2][y]) * 65536;
-              s += (long long)__float2int_rn(v[1][y]) * 16777216;
-              s += (long long)__float2int_rn(v[0][y]) << 32;
-              acc[x + y] = s;
+              long long s;
+              if constexpr (S == 7)
+                s = (long long)__float2int_rn(v[4][y]) * 16 + __float2int_rn(0.0625f * fmaf(v[6][y], 0.00390625f, v[5][y]));
+              else
+                s = __float2int_rn(fmaf(v[5][y], 0.00390625f, v[4][y]));
+              s += (long long)__float2int_rn(v[3][y]) << (8 + fine);
+              s += (long long)__float2int_rn(v[2][y]) << (16 + fine);
+              s += (long long)__float2int_rn(v[1][y]) << (24 + fine);
+              s += (long long)__float2int_rn(v[0][y]) << (32 + fine);
+              acc[x + y] += s;
             }
           }
         tc_fence_before();
@@ -435,8 +469,8 @@ __global__ void __launch_bounds__(kDgThreads, 1)
       }
       const int r = blk * kTcRows + q * 32 + lane;
       if (r >= g.R) continue;
-      // value = acc * 2^(rowexp + colexp - 2090)
-      const int er = g.rowexp[r] - 2090;
+      // value = acc * 2^(rowexp + colexp - 2090 - fine)
+      const int er = g.rowexp[r] - 2090 - fine;
       const int n0 = nt * BN + half * hc;
       const int64_t o0 = (int64_t)r * N + n0;
       // pairs of columns by 16-byte accesses where rows keep the alignment

@@ -69,6 +69,59 @@ def test_digit_products(built, M, N, D, width, flat, sparse):
     assert np.max(np.abs(G - Go)) <= eG + 1e-13 * np.max(np.abs(Go)), (np.max(np.abs(G - Go)), eG)
 
 
+@pytest.mark.parametrize("M,N,D,width", [(129, 5, 200, 20), (300, 16, 257, 200)])
+def test_digit_products_residual(built, M, N, D, width):
+    """Data that X reproduces to 1e-4: the residual's error is
+    that of 56-bit operands (_bounds' 48-bit one by 2^-8, and the roundings
+    of the sum and of the difference), and the gradient's what it grows to in
+    F^T.R with its 48 bits of the small R.  The reference has at least 64
+    bits of mantissa."""
+    import pqdts_gb300 as pq
+
+    inst = _instance(M, N, D, width, False, seed=M)
+    rng = np.random.default_rng(6)
+    X = rng.random((M, N)) + 0.1
+    X = np.asfortranarray(X / X.sum(1, keepdims=True))
+    F = inst.dense_F()
+    inst.P = F @ X * (1 + 1e-4 * rng.standard_normal((D, N)))
+    inst.gamma = 0.0
+    with pq.Solver(0) as s:
+        s.set_instance(inst, pq.MIXED)
+        s.set_x(X)
+        G = s.dL()
+    Fl = F.astype(np.longdouble)
+    R = 2 * (Fl @ X.astype(np.longdouble) - inst.P)
+    exact = Fl.T @ R
+    fm, Kt = np.abs(F).max(), int((F != 0).sum(0).max())
+    eO = 16 * (width + 16) * 2.0 ** -55 * fm * X.max() + 2.0 ** -51 * np.abs(inst.P).max()
+    eG = 2 * np.abs(F).sum(0).max() * eO + 16 * (Kt + 16) * 2.0 ** -47 * fm * float(np.abs(R).max())
+    eG += 2.0 ** -51 * float(np.abs(exact).max())
+    err = float(np.max(np.abs(G - exact)))
+    assert err <= eG, (err, eG)
+
+
+@pytest.mark.parametrize("width,digits", [(8191, 1), (8192, 0)])
+def test_digit_products_widest(built, width, digits):
+    """Terms of one sign at the scales' limit up to the width that the 64-bit
+    sums hold; wider rows in double-FP32."""
+    import pqdts_gb300 as pq
+
+    inst = _instance(width, 2, 2, width, True, seed=4)
+    most = 1 - 2.0 ** -53
+    inst.band_val[:] = most
+    inst.gamma = 0.0
+    X = np.full((width, 2), most, order="F")
+    with pq.Solver(0) as s:
+        s.set_instance(inst, pq.MIXED)
+        assert s.get_option("sched.dg_fwd") == digits
+        s.set_x(X)
+        G = s.dL()
+    R = 2 * (width - inst.P)
+    exact = np.broadcast_to(R.sum(0), (width, 2))
+    # the double-FP32 sums: 2^-47 of the sum so far for each of 2^13 terms
+    assert np.allclose(G, exact, rtol=2.0 ** -34, atol=0), np.abs(G / exact - 1).max()
+
+
 def test_digit_products_not_finite(built):
     """A NaN or an infinity in X reaches exactly the entries whose sums hold
     it: the rows of F with X's row in their band, then the columns of F with
