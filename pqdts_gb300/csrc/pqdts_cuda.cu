@@ -882,7 +882,8 @@ static void rebuild(Ctx& c, double* X, const double* saved, int32_t* chg) {
 }
 
 // Column chains (k_colchain's OP) of B stacked inputs: a block a chain while that leaves
-// an SM at most two blocks and the chain is long enough to pay for the guess
+// an SM at most two blocks (three with the paired dots of OP 2, in sum 304 and
+// 456) and the chain is long enough to pay for the guess
 // (two chains of 1000 terms a column, 200 blocks: 39 us either way; one: 29
 // against 39 by warps), a warp a chain otherwise.  advance: the CG's scalars
 // follow (OP 2 into SC_RZ, SC_RR).
@@ -1167,7 +1168,6 @@ static double op_L(Ctx& c) {
   if (!c.fullspace) rebuild_x(c);
   if (c.L_ver == c.xver) return c.L_cache;
   ensure_R(c);
-  const int D = (int)c.h.D, N = (int)c.h.N;
   residual_rows(c, c.R.p, 0.5, 1);
   objective_combine(c, c.X.p, 1);
   double L;
@@ -2144,8 +2144,6 @@ static void project_rows(Ctx& c, const double* X, const double* S, const double*
 // Candidates X + alpha_b*S (b < B) projected the way the stage requires and
 // rebuilt as L does, their objectives and (stage 2) xmin into c.pin.
 static void eval_candidates(Ctx& c, const double* al, int B, bool stage2, double* L, double* xmin) {
-  const int M = (int)c.h.M, N = (int)c.h.N;
-  const int64_t MN = (int64_t)M * N;
   CK(cudaMemcpyAsync(c.alphas.p, al, B * sizeof(double), cudaMemcpyHostToDevice, c.st));
   if (stage2) {
     Scope s(c.timers, "doproj2");
