@@ -665,7 +665,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
     c.tidx.upload(h.tidx.data(), h.tidx.size(), c.st, &c.h2d);
     c.tval.upload(h.tval.data(), h.tval.size(), c.st, &c.h2d);
   }
-  k_bdiag<<<cdiv(M, 32), 32, 0, c.st>>>(bands_of(c), c.tval.p, h.gam, c.bdiag.p);
+  k_bdiag<<<cdiv(M, 32), kBdiagThreads, 0, c.st>>>(bands_of(c), c.tval.p, h.gam, c.bdiag.p);
   post_launch(c);
   c.maxr.alloc(M);
   k_initial_maxr<<<cdiv(M, 32), 32, 0, c.st>>>(maxr_state, (int)M, (int)N, c.maxr.p);

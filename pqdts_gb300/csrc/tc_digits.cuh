@@ -249,13 +249,6 @@ __device__ __forceinline__ double dg_value(long long t, int e) {
                                           ((unsigned long long)t & 0x8000000000000000ull)));
 }
 
-// 2 x by its bits where x is normal.
-__device__ __forceinline__ double dg_twice(double x) {
-  const long long b = __double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7ff);
-  return (unsigned)(e - 1) < 2045u ? __longlong_as_double(b + (1ll << 52)) : x + x;
-}
-
 // Operands and results of one digit product.
 struct DgArgs {
   const int32_t *kb, *nch;           // K window of each 128-row block of A
@@ -501,7 +494,7 @@ __global__ void __launch_bounds__(kDgThreads, 1)
           const double2 p = load(g.P + o);
           v.x -= p.x;
           v.y -= p.y;
-          if (MODE == 0) v = make_double2(dg_twice(v.x), dg_twice(v.y));
+          if (MODE == 0) v = make_double2(twice(v.x), twice(v.y));
           store(g.out + o, v);
         } else {
           if (g.c2gam != 0.0) {
