@@ -635,6 +635,11 @@ static bool tc_wanted(const Ctx& c) {
   return major == 10;
 }
 
+// About eight blocks an SM for nb tiles, up to 16 a tile.
+static dim3 tile_build_grid(int64_t nb) {
+  return dim3((unsigned)nb, (unsigned)std::max<int64_t>(1, std::min<int64_t>(16, 8 * 152 / nb)));
+}
+
 // The problem's arrays on the device (maxr_state: the seeded stream before
 // the first maxr's draws) and the work buffers.
 static void setup_device(Ctx& c, uint64_t maxr_state) {
@@ -767,7 +772,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
     c.ftile_hi.upload(hi.data(), nb, c.st, &c.h2d);
     c.ftile_off.upload(off.data(), nb + 1, c.st, &c.h2d);
     c.ftile.alloc(std::max<int64_t>(off[nb], 1));
-    k_ftile_build<<<(unsigned)nb, 256, 0, c.st>>>(bands_of(c), c.tval.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p,
+    k_ftile_build<<<tile_build_grid(nb), 256, 0, c.st>>>(bands_of(c), c.tval.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p,
                                                    c.ftile.p);
     post_launch(c);
     c.ccnt.alloc((size_t)N * (cdiv(D, 32) + 1));
@@ -802,7 +807,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
     c.fwtile_hi.upload(hi.data(), nb, c.st, &c.h2d);
     c.fwtile_off.upload(off.data(), nb + 1, c.st, &c.h2d);
     c.fwtile.alloc(std::max<int64_t>(off[nb], 1));
-    k_fwtile_build<<<(unsigned)nb, 256, 0, c.st>>>(bands_of(c), c.fval.p, c.fwtile_lo.p, c.fwtile_hi.p,
+    k_fwtile_build<<<tile_build_grid(nb), 256, 0, c.st>>>(bands_of(c), c.fval.p, c.fwtile_lo.p, c.fwtile_hi.p,
                                                     c.fwtile_off.p, c.fwtile.p);
     post_launch(c);
     c.xcmask.alloc((size_t)kBatchLS * N * cdiv(M, 32));
