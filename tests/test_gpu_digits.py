@@ -122,6 +122,27 @@ def test_digit_products_widest(built, width, digits):
     assert np.allclose(G, exact, rtol=2.0 ** -34, atol=0), np.abs(G / exact - 1).max()
 
 
+@pytest.mark.parametrize("D,digits", [(2**17 - 1, 1), (2**17, 0)])
+def test_digit_products_tallest(built, D, digits):
+    """The same for F^T.R and the height of F's columns."""
+    import pqdts_gb300 as pq
+
+    inst = _instance(2, 2, D, 2, True, seed=4)
+    most = 1 - 2.0 ** -53
+    inst.band_val[:] = most
+    inst.gamma = 0.0
+    X = np.full((2, 2), most, order="F")
+    with pq.Solver(0) as s:
+        s.set_option("autotune", 0)
+        s.set_instance(inst, pq.MIXED)
+        assert s.get_option("sched.dg_fwd") == 1 and s.get_option("sched.dg_trans") == digits
+        s.set_x(X)
+        G = s.dL()
+    exact = np.broadcast_to((2 * (2 - inst.P)).sum(0), (2, 2))
+    # the double-FP32 sums: 2^-47 of the sum so far for each of 2^17 terms
+    assert np.allclose(G, exact, rtol=2.0 ** -30, atol=0), np.abs(G / exact - 1).max()
+
+
 def test_digit_products_not_finite(built):
     """A NaN or an infinity in X reaches exactly the entries whose sums hold
     it: the rows of F with X's row in their band, then the columns of F with
