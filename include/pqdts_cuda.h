@@ -88,9 +88,10 @@ int pqdts_cuda_kernel_launches(pqdts_ctx* ctx, int64_t* count);
  *   "df_products" -1 (default, auto): the mixed path's gradient F^T.R
  *              and its objective checks (residual F.X - P) by exact digits
  *              on the tensor cores where those are in use ("tensor_cores")
- *              and F is finite (48 bits of each row's and column's scale,
- *              error ~sqrt(K) * 2^-47 of their product for K terms), else as
- *              1: in double-FP32
+ *              and F is finite (operands to 56 bits of a scale for each 256
+ *              terms of a row or column; sums that are small beside their
+ *              scales are formed as under 1, so that no entry is less
+ *              accurate than there), else as 1: in double-FP32
  *              (pairs of FP32 numbers, ~sqrt(K) * 2^-48 relative to the
  *              sum of the K terms' magnitudes) on the CUDA cores; 0: native
  *              FP64.  Takes

@@ -300,14 +300,17 @@ struct TcOperand {
 };
 
 // Band operand of the digit products: the digits of a TcOperand's row blocks
-// (same K windows), each row's exponent, the product's N tile width and tile
+// (same K windows), each row's scales, the product's N tile width and tile
 // lists, and the B operand's map for that width.
 struct DgOperand {
   DBuf<uint16_t> dig;
-  DBuf<int> rowexp;
+  DBuf<int> rowexp, rowall;
   CUtensorMap map_a, map_b;
   TcSched sched;
   int bn = 0, stages = 0;
+  int groups = 0;     // of K that a row block's window meets, at most
+  int fine = 0;       // bits of the sums below 2^-48 of the scales
+  float floor = 0.f;  // sum of magnitudes below which an output is formed again
 };
 
 // CG work vectors of one precision.
@@ -403,7 +406,8 @@ struct pqdts_ctx {
   bool dg_fwd = false, dg_trans = false;
   pqdts::DgOperand dgF, dgFt;
   pqdts::DBuf<uint16_t> dg_x, dg_r;
-  pqdts::DBuf<int> dg_colexp;
+  pqdts::DBuf<int> dg_col, dg_colexp;  // k_dg_columns (one more: whether dg_redo marks any)
+  pqdts::DBuf<uint8_t> dg_redo;   // outputs left to the double-FP32 kernels
   bool exact = true;  // FP64: every reduction in the oracle's order
   pqdts::DBuf<int> ipart;
   pqdts::DBuf<long long> icount;
@@ -601,9 +605,14 @@ static void check_products(Ctx& c) {
 // Band rows per block of the double-FP32 products: the most of 8, 4, 2
 // that still gives >= 40 warps per SM to cover the operand loads' latency
 // (measured: M=2000, N=200, D=4000 runs best at 4 rows for F.X and 2 for
-// F^T.R; M=10^4, N=10^3, D=2*10^4 at 8); rbopt > 0: that, as 2/4/8.
-static int df_rows_per_block(int64_t rows, int N, int rbopt, int sms) {
+// F^T.R; M=10^4, N=10^3, D=2*10^4 at 8); rbopt > 0: that, as 2/4/8.  part:
+// only the outputs that a digit product left are formed; then an eighth of
+// the blocks or so have any, each a long chain, and the smaller blocks that
+// fill the SMs all the same are faster (M = 5003, N = 501
+// mid-solve: F^T.R's 1.2-1.4 ms -> 0.56, F.X's 0.58 -> 0.61).
+static int df_rows_per_block(int64_t rows, int N, int rbopt, int sms, bool part) {
   if (rbopt > 0) return rbopt >= 8 ? 8 : (rbopt >= 4 ? 4 : 2);
+  if (part) rows /= 8;
   const int64_t wpr = cdiv(N, 32);
   for (int rb : {8, 4})
     if ((rows + rb - 1) / rb * wpr >= (int64_t)40 * sms) return rb;
@@ -611,15 +620,15 @@ static int df_rows_per_block(int64_t rows, int N, int rbopt, int sms) {
 }
 
 template <int MODE>
-static void launch_fwd_df(Ctx& c, double* R, const uint32_t* xmask) {
+static void launch_fwd_df(Ctx& c, double* R, const uint32_t* xmask, const DfRedo& redo) {
   const int N = (int)c.h.N, D = (int)c.h.D;
-  const int rb = df_rows_per_block(D, N, c.df_rows, c.num_sms);
+  const int rb = df_rows_per_block(D, N, c.df_rows, c.num_sms, redo.bits != nullptr);
   const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
   const dim3 grid(cdiv(D, rb), cdiv(N, threads));
   DevBands bd = bands_of(c);
-  if (rb == 8) k_fwd_df<MODE, 8><<<grid, threads, 0, c.st>>>(bd, c.fdf.p, c.xdf.p, c.P.p, R, xmask);
-  else if (rb == 4) k_fwd_df<MODE, 4><<<grid, threads, 0, c.st>>>(bd, c.fdf.p, c.xdf.p, c.P.p, R, xmask);
-  else k_fwd_df<MODE, 2><<<grid, threads, 0, c.st>>>(bd, c.fdf.p, c.xdf.p, c.P.p, R, xmask);
+  if (rb == 8) k_fwd_df<MODE, 8><<<grid, threads, 0, c.st>>>(bd, c.fdf.p, c.xdf.p, c.P.p, R, xmask, redo);
+  else if (rb == 4) k_fwd_df<MODE, 4><<<grid, threads, 0, c.st>>>(bd, c.fdf.p, c.xdf.p, c.P.p, R, xmask, redo);
+  else k_fwd_df<MODE, 2><<<grid, threads, 0, c.st>>>(bd, c.fdf.p, c.xdf.p, c.P.p, R, xmask, redo);
   post_launch(c);
 }
 
@@ -717,7 +726,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
     const auto widest = [](const std::vector<int32_t>& w) { return w.empty() ? 0 : *std::max_element(w.begin(), w.end()); };
     c.dg_fwd = c.df_option < 0 && c.f_finite && widest(h.fw) < kDgMaxFwd && tc_wanted(c);
     c.dg_trans = c.dg_fwd && c.t_contiguous && widest(h.tw) < kDgMaxTrans;
-    if (c.df_fwd && !c.dg_fwd) {
+    if (c.df_fwd) {
       c.fdf.alloc(nnz);
       k_split_df<<<elem_grid(nnz), 256, 0, c.st>>>(c.fval.p, nnz, 1.0, c.fdf.p);
       post_launch(c);
@@ -726,7 +735,7 @@ static void setup_device(Ctx& c, uint64_t maxr_state) {
       c.fdf.release();
       c.xdf.release();
     }
-    if (c.df_trans && !c.dg_trans) {
+    if (c.df_trans) {
       c.tdf.alloc(nnz);
       k_split_df<<<elem_grid(nnz), 256, 0, c.st>>>(c.tval.p, nnz, 1.0, c.tdf.p);
       post_launch(c);
@@ -1011,29 +1020,32 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
 
 
 // The mixed path's digit products read `rows` x N doubles of B as digits of
-// each column's scale: the columns' exponents, then the transposed digits.
-template <int S>
+// each column's scales: the scales, then the transposed digits.
 static void dg_split(Ctx& c, const double* B, int rows, int64_t ld, DBuf<uint16_t>& dig) {
   const int N = (int)c.h.N;
-  CK(cudaMemsetAsync(c.dg_colexp.p, 0, N * sizeof(int), c.st));
-  // ~4 blocks per SM, at least 64 rows each
-  const int shares = std::max(1, std::min(cdiv(rows, 64), cdiv((int64_t)4 * c.num_sms, cdiv(N, 32))));
-  k_dg_colexp<<<dim3(cdiv(N, 32), shares), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p);
+  CK(cudaMemsetAsync(c.dg_col.p, 0, (3 * (size_t)N + 1) * sizeof(int), c.st));
+  k_dg_columns<<<dim3(cdiv(N, 32), cdiv(rows, kDgGroup)), 256, 0, c.st>>>(B, rows, N, c.dg_col.p, c.dg_colexp.p);
   post_launch(c);
-  k_dg_split_t<S><<<dim3(cdiv(rows, 64), cdiv(N, 32)), 256, 0, c.st>>>(B, rows, N, c.dg_colexp.p, ld, dig.p);
+  k_dg_split_t<<<dim3(cdiv(rows, 64), cdiv(N, 32)), 256, 0, c.st>>>(B, rows, N, c.dg_col.p, c.dg_colexp.p, ld, dig.p);
   post_launch(c);
 }
 
 // One digit product: op's rows (`rows` of F or F^T) times the digits in
-// place, B their FP64 values; see k_dg_band_product for the modes.
+// place, B their FP64 values; see k_dg_band_product for the modes.  Returns
+// the outputs that are left to the double-FP32 kernels.
 template <int MODE>
-static void dg_product(Ctx& c, DgOperand& op, TcOperand& win, int rows, const double* B, double* out, double* out2,
+static DfRedo dg_product(Ctx& c, DgOperand& op, TcOperand& win, int rows, const double* B, double* out, double* out2,
                        const double* V, double c2gam) {
   DgArgs g;
   g.kb = win.kb.p;
   g.nch = win.nch.p;
   g.rowexp = op.rowexp.p;
+  g.rowall = op.rowall.p;
   g.colexp = c.dg_colexp.p;
+  g.col = c.dg_col.p;
+  g.groups = op.groups;
+  g.K = (int)(MODE == 4 ? c.h.D : c.h.M);
+  g.fine = op.fine;
   g.sched_off = op.sched.off.p;
   g.sched_tile = op.sched.tile.p;
   g.R = rows;
@@ -1045,6 +1057,10 @@ static void dg_product(Ctx& c, DgOperand& op, TcOperand& win, int rows, const do
   g.c2gam = c2gam;
   g.out = out;
   g.out2 = out2;
+  g.floor = op.floor;
+  g.redo = c.dg_redo.p;
+  g.pitch = cdiv(c.h.N, 8);
+  g.any = c.dg_col.p + 3 * c.h.N;
   g.f = bands_of(c);
   g.val = MODE == 4 ? c.tval.p : c.fval.p;
   g.B = B;
@@ -1052,32 +1068,35 @@ static void dg_product(Ctx& c, DgOperand& op, TcOperand& win, int rows, const do
   g.wait_ns = c.tc_wait_ns;
   k_dg_band_product<MODE><<<op.sched.grid, kDgThreads, kDgRing + 1024, c.st>>>(op.map_a, op.map_b, g);
   post_launch(c);
+  return {g.redo, g.pitch, g.any};
 }
 
 // Residual of X (FP64, M x N) to FP64 accuracy without the FP64 pipe: MODE 0
-// R = 2*(F.X - P), MODE 3 R = F.X - P.  By digits on the tensor cores where
-// those are in use, else in double-FP32.
+// R = 2*(F.X - P), MODE 3 R = F.X - P.  In double-FP32, or where digits are in
+// use on the tensor cores, and in double-FP32 then only where a sum is so
+// small beside its operands' scales that the digits hold it less accurately.
 template <int MODE>
 static void fwd_df(Ctx& c, const double* X, double* R) {
   const int64_t MN = c.h.M * c.h.N;
+  DfRedo redo;
   if (c.dg_fwd) {
-    dg_split<kDgFwd>(c, X, (int)c.h.M, c.tc_mp, c.dg_x);
-    dg_product<MODE>(c, c.dgF, c.tcF, (int)c.h.D, X, R, nullptr, nullptr, 0.0);
-    return;
+    dg_split(c, X, (int)c.h.M, c.tc_mp, c.dg_x);
+    redo = dg_product<MODE>(c, c.dgF, c.tcF, (int)c.h.D, X, R, nullptr, nullptr, 0.0);
   }
   require(c.xdf.p, "xdf");
-  k_split_df<<<elem_grid(MN), 256, 0, c.st>>>(X, MN, 1.0, c.xdf.p);
+  k_split_df<<<elem_grid(MN), 256, 0, c.st>>>(X, MN, 1.0, c.xdf.p, redo.any);
   post_launch(c);
   const uint32_t* xm = nullptr;
   if (c.mask_option != 0 && c.f_finite) {
     // X's row-occupancy masks: the product visits only rows where a warp's
     // columns are non-zero
     const int M = (int)c.h.M, ng = cdiv(c.h.N, 32), nseg = cdiv(M, 32);
-    k_row_masks<double><<<dim3(cdiv((int64_t)ng * nseg * 32, 256), 1), 256, 0, c.st>>>(X, 0, M, (int)c.h.N, c.xmask.p);
+    k_row_masks<double><<<dim3(cdiv((int64_t)ng * nseg * 32, 256), 1), 256, 0, c.st>>>(X, 0, M, (int)c.h.N, c.xmask.p,
+                                                                                                redo.any);
     post_launch(c);
     xm = c.xmask.p;
   }
-  launch_fwd_df<MODE>(c, R, xm);
+  launch_fwd_df<MODE>(c, R, xm, redo);
 }
 
 // Residual row sums of B stacked residuals, each scale * R, into srow.
@@ -1305,27 +1324,27 @@ static void op_dL(Ctx& c) {
       post_launch(c);
     }
   } else if (c.df_trans) {
-    // mixed path, digits or double-FP32: full-space gradient into Gf (and
-    // G), then the reduced one from it
+    // mixed path, digits and double-FP32 (as fwd_df): full-space gradient into
+    // Gf (and G), then the reduced one from it
     ensure_R(c);
     const int D = (int)c.h.D;
     double* g = c.fullspace ? c.G.p : nullptr;
     const double c2g = 2.0 * c.h.gam;
+    DfRedo redo;
     if (c.dg_trans) {
-      dg_split<kDgTrans>(c, c.R.p, D, c.tc_dp, c.dg_r);
-      dg_product<4>(c, c.dgFt, c.tcFt, M, c.R.p, c.Gf.p, g, c.X.p, c2g);
-    } else {
-      k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p);
-      post_launch(c);
-      const int rb = df_rows_per_block(M, N, c.df_rows, c.num_sms);
-      const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
-      const dim3 grid(cdiv(M, rb), cdiv(N, threads));
-      DevBands bd = bands_of(c);
-      if (rb == 8) k_trans_df<8><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
-      else if (rb == 4) k_trans_df<4><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
-      else k_trans_df<2><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p);
-      post_launch(c);
+      dg_split(c, c.R.p, D, c.tc_dp, c.dg_r);
+      redo = dg_product<4>(c, c.dgFt, c.tcFt, M, c.R.p, c.Gf.p, g, c.X.p, c2g);
     }
+    k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p, redo.any);
+    post_launch(c);
+    const int rb = df_rows_per_block(M, N, c.df_rows, c.num_sms, redo.bits != nullptr);
+    const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
+    const dim3 grid(cdiv(M, rb), cdiv(N, threads));
+    DevBands bd = bands_of(c);
+    if (rb == 8) k_trans_df<8><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
+    else if (rb == 4) k_trans_df<4><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
+    else k_trans_df<2><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
+    post_launch(c);
     if (!c.fullspace) {
       k_reduced_from_full<<<M, std::min(256, std::max(32, cdiv(N, 32) * 32)), 0, c.st>>>(c.Gf.p, c.maxr.p, N, c.G.p);
       post_launch(c);
@@ -1539,16 +1558,17 @@ static void make_map_digits(CUtensorMap* m, const void* base, uint64_t inner, ui
 }
 
 // N tile width of a digit product over A's row blocks: the one of 64, 48,
-// 32, 16 (their six or seven levels fit tensor memory) with the least estimated
-// time, waves of tiles x the cycles of a K chunk (21 or 28 digit pairs x BN / 2
-// a K slice of arithmetic and ~45 of start-up for each of the 11 MMAs, two
-// slices), so narrow tiles are taken only to fill the SMs.
-static int dg_tile_n(const Ctx& c, const TcOperand& A, int digits) {
+// 32, 16 (their seven levels and the magnitudes fit tensor memory) with the
+// least estimated time, waves of tiles x the cycles of a K chunk (28 digit
+// pairs and the magnitudes x BN / 2 a K slice of arithmetic and ~45 of
+// start-up for each of the 14 MMAs, two slices), so narrow tiles are taken
+// only to fill the SMs.
+static int dg_tile_n(const Ctx& c, const TcOperand& A) {
   const int N = (int)c.h.N;
   int best = 16;
   int64_t least = INT64_MAX;
   for (int bn : {64, 48, 32, 16}) {
-    const int64_t t = (int64_t)(digits * (digits + 1) / 2 * bn + 990) * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
+    const int64_t t = (int64_t)(29 * bn + 2 * 45 * 14) * cdiv((int64_t)cdiv(N, bn) * A.blocks, c.num_sms);
     if (t < least) {
       least = t;
       best = bn;
@@ -1562,16 +1582,24 @@ static int dg_tile_n(const Ctx& c, const TcOperand& A, int digits) {
 static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf<uint16_t>& dig_b, int64_t K,
                          int64_t ld) {
   const int N = (int)c.h.N, rows = win.blocks * kTcRows;
-  const int S = trans ? kDgTrans : kDgFwd;
+  const int S = kDgSlices;
+  const std::vector<int32_t>& widths = trans ? c.h.tw : c.h.fw;
+  const int terms = widths.empty() ? 0 : *std::max_element(widths.begin(), widths.end());
+  op.fine = dg_fine(terms);
+  op.groups = win.kmax / kDgGroup + 2;
+  op.floor = dg_floor(terms, op.groups, op.fine);
   op.dig.alloc((size_t)S * rows * win.kmax);
-  op.rowexp.alloc(rows);
+  op.rowexp.alloc((size_t)rows * op.groups);
+  op.rowall.alloc(rows);
   dig_b.alloc((size_t)S * N * ld);
   if (trans)
-    k_dg_band<true><<<rows, 256, 0, c.st>>>(bands_of(c), c.tval.p, win.kb.p, rows, win.kmax, op.dig.p, op.rowexp.p);
+    k_dg_band<true><<<rows, 256, 0, c.st>>>(bands_of(c), c.tval.p, win.kb.p, rows, win.kmax, op.groups,
+                                             op.dig.p, op.rowexp.p, op.rowall.p);
   else
-    k_dg_band<false><<<rows, 256, 0, c.st>>>(bands_of(c), c.fval.p, win.kb.p, rows, win.kmax, op.dig.p, op.rowexp.p);
+    k_dg_band<false><<<rows, 256, 0, c.st>>>(bands_of(c), c.fval.p, win.kb.p, rows, win.kmax, op.groups,
+                                             op.dig.p, op.rowexp.p, op.rowall.p);
   post_launch(c);
-  op.bn = dg_tile_n(c, win, S);
+  op.bn = dg_tile_n(c, win);
   const uint32_t stage = S * (kTcRows + (uint32_t)op.bn) * kTcRowBytes;
   op.stages = std::min<int>(kDgMaxStages, (int)(kDgRing / stage));
   make_map_digits(&op.map_a, op.dig.p, win.kmax, rows, win.kmax, kTcRows, S);
@@ -1604,7 +1632,9 @@ static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf
 
 static void setup_dg(Ctx& c) {
   if (!c.dg_fwd) return;
-  c.dg_colexp.alloc(c.h.N);
+  c.dg_col.alloc(3 * (size_t)c.h.N + 1);
+  c.dg_colexp.alloc((size_t)cdiv(std::max(c.h.D, c.h.M), kDgGroup) * c.h.N);
+  c.dg_redo.alloc((size_t)std::max(c.h.D, c.h.M) * cdiv(c.h.N, 8));
   for (auto k : {k_dg_band_product<0>, k_dg_band_product<3>, k_dg_band_product<4>})
     CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDgRing + 1024));
   setup_digits(c, c.dgF, c.tcF, false, c.dg_x, c.h.M, c.tc_mp);

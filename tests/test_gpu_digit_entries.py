@@ -1,0 +1,82 @@
+"""The mixed path's gradient and residual products entry by entry: a sum that
+is small beside the scales of its row of F and its column of X (or R) is as
+accurate as double-FP32 leaves it, however the operands' magnitudes spread."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _spread(M, N, D, width, seed):
+    """Bands of `width` columns that fall off by 2^-30 from their middle, and
+    (D, N) and (M, N) arrays that fall off by 2^-50 from a diagonal, with a
+    column and a tenth of the entries zero."""
+    from pqdts_gb300.synth import Instance
+
+    rng = np.random.default_rng(seed)
+    lo = np.round(np.linspace(0, M - width, D)).astype(np.int64)
+    u = np.linspace(-1, 1, width)
+    val = (rng.random((D, width)) + 0.5) * 2.0 ** (-30 * u * u)
+
+    def profile(rows):
+        away = np.abs(np.linspace(0, 1, rows)[:, None] - np.linspace(0, 1, N)[None, :])
+        a = (rng.random((rows, N)) + 0.5) * 2.0 ** (-50 * away)
+        a[rng.random((rows, N)) < 0.1] = 0.0
+        a[:, N // 2] = 0.0
+        return a
+
+    inst = Instance(M, N, D, 0.0, 1e-6, lo, lo + width - 1, val.ravel(), profile(D))
+    return inst, np.asfortranarray(profile(M))
+
+
+def _dense(inst):
+    return inst.dense_F().astype(np.longdouble)
+
+
+def _check(G, exact, size, K, products):
+    """Double-FP32 rounds a sum of K terms by ~0.2 sqrt(K) 2^-48 of its terms'
+    magnitudes (rms): within 40 times that for each of the products."""
+    bound = products * 8 * np.sqrt(K) * 2.0 ** -48 * size
+    err = np.abs(G - exact)
+    assert np.all(err <= bound), float(np.max(err[size > 0] / bound[size > 0]))
+
+
+SIZES = [(300, 27, 555, 60), (900, 40, 700, 300), (129, 70, 400, 100), (200, 2, 3000, 40)]
+
+
+@pytest.mark.parametrize("M,N,D,width", SIZES)
+def test_gradient_entries(built, M, N, D, width):
+    """F^T.R alone: X = 0, so R = -2 P exactly."""
+    import pqdts_gb300 as pq
+
+    inst, _ = _spread(M, N, D, width, seed=D)
+    F = _dense(inst)
+    with pq.Solver(0) as s:
+        s.set_option("autotune", 0)
+        s.set_instance(inst, pq.MIXED)
+        assert s.get_option("sched.dg_trans") == 1
+        s.set_x(np.zeros((M, N), order="F"))
+        G = s.dL()
+    K = int((F != 0).sum(0).max())
+    _check(G, F.T @ (-2 * inst.P), F.T @ (2 * inst.P), K, 1)
+
+
+@pytest.mark.parametrize("M,N,D,width", SIZES)
+def test_residual_entries(built, M, N, D, width):
+    """F.X, then F^T of it (P = 0; every term positive)."""
+    import pqdts_gb300 as pq
+
+    inst, X = _spread(M, N, D, width, seed=M)
+    inst.P = np.zeros((D, N))
+    F = _dense(inst)
+    with pq.Solver(0) as s:
+        s.set_option("autotune", 0)
+        s.set_instance(inst, pq.MIXED)
+        assert s.get_option("sched.dg_fwd") == 1
+        s.set_x(X)
+        G, L = s.dL(), s.L()
+    O = F @ X
+    exact = F.T @ (2 * O)
+    K = max(width, int((F != 0).sum(0).max()))
+    _check(G, exact, exact, K, 2)
+    assert abs(L - float((O * O).sum())) <= 16 * np.sqrt(K) * 2.0 ** -48 * L
