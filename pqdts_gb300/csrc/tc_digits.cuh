@@ -103,9 +103,9 @@ __device__ __forceinline__ int dg_exponent(double v) { return (int)((__double_as
 __device__ __forceinline__ int dg_scale(double v) { return nonzero(v) ? max(1, dg_exponent(v)) : 0; }
 
 // The S digits (bf16 bit patterns, most significant first) of v, whose biased
-// exponent is at most emax >= 1 (or v = 0): v = 2^(emax - 1021 - 8 S) t, t = v's mantissa
-// shifted to the scale's 8 S bits, rounded half away from zero; each byte of
-// t + 0x8080...80 is a digit + 128.  Then |v| 2^(1021 - eall), below 1/2 (eall:
+// exponent is at most emax >= 1 (or v = 0): v = 2^(emax - 1021 - 8 S) t, t =
+// v's mantissa shifted to the scale's 8 S bits, rounded half away from zero;
+// each byte of t + 0x8080...80 is a digit + 128.  Then |v| 2^(1021 - eall), below 1/2 (eall:
 // the largest exponent of the whole row or column), truncated to bf16.
 __device__ __forceinline__ void dg_digits(double v, int emax, int eall, uint32_t (&d)[kDgSlices]) {
   constexpr int S = kDgDigits;
@@ -126,7 +126,7 @@ __device__ __forceinline__ void dg_digits(double v, int emax, int eall, uint32_t
     // 2^23 + byte as a float, minus 2^23 + 128: the digit, exactly
     d[q] = __float_as_uint(__fsub_rn(__uint_as_float(0x4b000000u | byte), 8388736.0f)) >> 16;
   }
-  const int be = dg_exponent(v) - eall + 125;
+  const int be = dg_exponent(v) - eall + 125;  // (subnormal: none)
   d[S] = be > 0 && dg_exponent(v) > 0 ? ((uint32_t)be << 7) | ((uint32_t)(b >> 45) & 0x7fu) : 0u;
 }
 

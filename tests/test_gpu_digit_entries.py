@@ -80,3 +80,26 @@ def test_residual_entries(built, M, N, D, width):
     K = max(width, int((F != 0).sum(0).max()))
     _check(G, exact, exact, K, 2)
     assert abs(L - float((O * O).sum())) <= 16 * np.sqrt(K) * 2.0 ** -48 * L
+
+
+def test_subnormal_scales(built):
+    """Columns of X whose largest magnitude is subnormal, against an F large
+    enough for a normal product: as in double-FP32 (which has no such
+    numbers)."""
+    import pqdts_gb300 as pq
+
+    M, N, D, width = 140, 5, 150, 33
+    inst, _ = _spread(M, N, D, width, seed=3)
+    rng = np.random.default_rng(4)
+    inst.P = np.zeros((D, N))
+    X = np.asfortranarray(np.ldexp(rng.integers(1, 1025, (M, N)).astype(float), -1060))
+    inst.band_val = np.ldexp(rng.random(D * width) + 0.5, 100)
+    G = []
+    for df in (-1, 1):
+        with pq.Solver(0) as s:
+            s.set_option("autotune", 0)
+            s.set_option("df_products", df)
+            s.set_instance(inst, pq.MIXED)
+            s.set_x(X)
+            G.append(s.dL())
+    assert np.array_equal(G[0], G[1])
