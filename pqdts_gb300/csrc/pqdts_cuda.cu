@@ -575,12 +575,12 @@ static void read_back(Ctx& c, const double* dev, int count) {
 
 // After a read-back of the scalars: a tensor-core kernel whose bounded
 // barrier wait ran out has set SC_TCERR.  The flag is cleared (the kernels
-// freed their tensor memory and stored nothing, the context stays usable)
-// and the call fails with PQDTS_E_CUDA.
+// freed their tensor memory; what they were to write is undefined, the
+// context stays usable) and the call fails with PQDTS_E_CUDA.
 static void throw_tc_error(Ctx& c) {
   CK(cudaMemsetAsync(c.sc.p + SC_TCERR, 0, sizeof(double), c.st));
   CK(cudaStreamSynchronize(c.st));
-  // what the product was to write is not there
+  // results held for this X are not there
   c.R_ver = c.G_ver = c.Gf_ver = c.L_ver = c.Graw_ver = -1;
   throw Err(PQDTS_E_CUDA, "tensor-core product: a barrier wait timed out");
 }
@@ -589,14 +589,14 @@ static void check_tc_error(Ctx& c) {
   if (c.pin[SC_TCERR] != 0.0) throw_tc_error(c);
 }
 
-// Waits for the stream; on a context whose gradient and objective products
-// run on the tensor cores, also checks that none of them gave up.
+// Waits for the stream; on a context with tensor-core products also checks
+// that none of them gave up.
 static void check_products(Ctx& c) {
-  constexpr int kAt = 48;  // scalars' place in the pinned buffer, past every other read-back
-  if (c.dg_fwd)
+  constexpr int kAt = 48;  // the flag's place in the pinned buffer, past every other read-back
+  if (c.tc_ready)
     CK(cudaMemcpyAsync(c.pin + kAt, c.sc.p + SC_TCERR, sizeof(double), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
-  if (c.dg_fwd && c.pin[kAt] != 0.0) throw_tc_error(c);
+  if (c.tc_ready && c.pin[kAt] != 0.0) throw_tc_error(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -1066,6 +1066,7 @@ static DfRedo dg_product(Ctx& c, DgOperand& op, TcOperand& win, int rows, const 
   g.B = B;
   g.err = c.sc.p + SC_TCERR;
   g.wait_ns = c.tc_wait_ns;
+  g.probe = c.tc_wait_probe;
   k_dg_band_product<MODE><<<op.sched.grid, kDgThreads, kDgRing + 1024, c.st>>>(op.map_a, op.map_b, g);
   post_launch(c);
   return {g.redo, g.pitch, g.any};
@@ -2657,21 +2658,24 @@ static void upload_colmajor(Ctx& c, const double* in, T* dev, int slot = 0) {
   post_launch(c);
 }
 
-// (waits for the stream)
+// (waits for the stream; products: the array is a product's result, and is not
+// written to `out` when the product gave up)
 template <typename T>
-static void download_colmajor(Ctx& c, const T* dev, double* out) {
+static void download_colmajor(Ctx& c, const T* dev, double* out, bool products = false) {
   const int M = (int)c.h.M, N = (int)c.h.N;
   const int64_t MN = (int64_t)M * N;
   if (MN <= kHostTranspose) {
     T* rm = small_stage<T>(c, 2);
     CK(cudaMemcpyAsync(rm, dev, MN * sizeof(T), cudaMemcpyDeviceToHost, c.st));
-    CK(cudaStreamSynchronize(c.st));
+    if (products) check_products(c);
+    else CK(cudaStreamSynchronize(c.st));
     for (int i = 0; i < M; ++i)
       for (int n = 0; n < N; ++n) out[i + (int64_t)n * M] = (double)rm[(size_t)i * N + n];
     return;
   }
   k_transpose<T, double><<<cdiv(M, 32) * cdiv(N, 32), 256, 0, c.st>>>(dev, M, N, c.Xc.p);
   post_launch(c);
+  if (products && c.tc_ready) check_products(c);
   CK(cudaMemcpyAsync(out, c.Xc.p, MN * sizeof(double), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
 }
@@ -3533,8 +3537,7 @@ int pqdts_cuda_dL(pqdts_ctx* c, double* G) {
   return guarded(c, [&] {
     pqdts::need_problem(*c);
     pqdts::op_dL(*c);
-    pqdts::download_colmajor(*c, c->G.p, G);
-    pqdts::check_products(*c);
+    pqdts::download_colmajor(*c, c->G.p, G, true);
   });
 }
 
@@ -3581,9 +3584,7 @@ int pqdts_cuda_BF32(pqdts_ctx* c, const double* V, double* HV) {
       pqdts::post_launch(*c);
     }
     pqdts::hvp32(*c, b, nullptr, false, nullptr);
-    CK(cudaMemcpyAsync(c->pin, c->sc.p, pqdts::SC_NSC * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    pqdts::download_colmajor(*c, b.Hp.p, HV);
-    pqdts::check_tc_error(*c);
+    pqdts::download_colmajor(*c, b.Hp.p, HV, true);
     c->d2h += M * N * 8;
   });
 }

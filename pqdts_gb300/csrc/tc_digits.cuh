@@ -359,6 +359,7 @@ struct DgArgs {
   const double *val, *B;
   double* err;
   uint64_t wait_ns;
+  int probe;
 };
 
 // Row r of F (TRANS: F^T) times column n of B in plain FP64: the result for
@@ -375,16 +376,18 @@ __device__ __noinline__ double dg_plain(const DgArgs& g, int r, int n) {
 
 // MODE 0: out = 2 (F.B - P); MODE 3: out = F.B - P (R = D rows of F);
 // MODE 4: F^T.B + the gamma stencil on V into out and / or out2 (R = M rows
-// of F^T; either may be null).  Every wait is bounded as in k_tc_band; a
-// wait that runs out sets *err and the CTA stores nothing more, lets the
-// copies and MMAs in flight finish and frees its tensor memory.
+// of F^T; either may be null).  Every wait is bounded as in k_tc_band, with
+// the same test hook; a wait that runs out sets *err and the CTA stores nothing
+// more (the tiles before are stored, and other CTAs' may be: the result is
+// undefined), lets the copies and MMAs in flight finish and frees its tensor
+// memory.
 template <int MODE>
 __global__ void __launch_bounds__(kDgThreads, 1)
     k_dg_band_product(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
                       const __grid_constant__ DgArgs g) {
   constexpr int S = kDgDigits;
   extern __shared__ uint8_t tc_smem_raw[];
-  __shared__ uint64_t bar_full[kDgMaxStages], bar_empty[kDgMaxStages], bar_accf, bar_acce, bar_fin;
+  __shared__ uint64_t bar_full[kDgMaxStages], bar_empty[kDgMaxStages], bar_accf, bar_acce, bar_fin, bar_probe;
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
   __shared__ int s_issued, s_consumed;
@@ -408,6 +411,7 @@ __global__ void __launch_bounds__(kDgThreads, 1)
     mbar_init(&bar_accf, 1);
     mbar_init(&bar_acce, 256);
     mbar_init(&bar_fin, 1);
+    mbar_init(&bar_probe, 1);
     s_abort = 0;
     s_issued = 0;
     s_consumed = 0;
@@ -427,6 +431,7 @@ __global__ void __launch_bounds__(kDgThreads, 1)
   if (warp == 0) {
     if (lane == 0) {
       int it = 0;
+      if (g.probe && !mbar_wait(&bar_probe, 0, g.wait_ns)) s_abort = 1;  // nothing arrives: runs out
       for (int j = j_begin; j < j_end && !s_abort; ++j) {
         const int t = g.sched_tile[j], nt = t % ntn, blk = t / ntn, kb = g.kb[blk];
         const int nk = kb >= 0 ? g.nch[blk] : 0;
