@@ -130,7 +130,8 @@ int pqdts_cuda_set_option(pqdts_ctx* ctx, const char* name, int64_t value);
  * (of their F.V product), "sched.tc_persistent" (kernel form),
  * "sched.df_fwd", "sched.df_trans" (double-FP32 residual / gradient
  * products in use, or their digit forms), "sched.dg_fwd", "sched.dg_trans"
- * (digit products in use), "sched.tc_screen" (line-search probe products on the
+ * (digit products in use), "sched.dg_bytes" (device memory that their operands
+ * hold), "sched.tc_screen" (line-search probe products on the
  * tensor cores), "graphs.captured" (graphs held). */
 int pqdts_cuda_get_option(pqdts_ctx* ctx, const char* name, int64_t* value);
 /* verbose = 1 prints the reference's stdout lines (iter, newton-pcg, line

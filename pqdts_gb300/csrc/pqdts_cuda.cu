@@ -311,6 +311,13 @@ struct DgOperand {
   int groups = 0;     // of K that a row block's window meets, at most
   int fine = 0;       // bits of the sums below 2^-48 of the scales
   float floor = 0.f;  // sum of magnitudes below which an output is formed again
+  void release() {
+    dig.release();
+    rowexp.release();
+    rowall.release();
+    sched.off.release();
+    sched.tile.release();
+  }
 };
 
 // CG work vectors of one precision.
@@ -1631,8 +1638,29 @@ static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf
   CK(cudaStreamSynchronize(c.st));  // the host vectors go out of scope
 }
 
+// Device memory that the digit products' operands hold.
+static int64_t dg_held(const Ctx& c) {
+  const DgOperand *a = &c.dgF, *b = &c.dgFt;
+  return (int64_t)(2 * (a->dig.cap + b->dig.cap + c.dg_x.cap + c.dg_r.cap) +
+                   4 * (a->rowexp.cap + b->rowexp.cap + a->rowall.cap + b->rowall.cap + c.dg_col.cap + c.dg_colexp.cap) +
+                   c.dg_redo.cap);
+}
+
+// What a problem does not use is given back: the operands are among the largest
+// arrays that a mixed one holds.
 static void setup_dg(Ctx& c) {
-  if (!c.dg_fwd) return;
+  if (!c.dg_trans) {
+    c.dgFt.release();
+    c.dg_r.release();
+  }
+  if (!c.dg_fwd) {
+    c.dgF.release();
+    c.dg_x.release();
+    c.dg_col.release();
+    c.dg_colexp.release();
+    c.dg_redo.release();
+    return;
+  }
   c.dg_col.alloc(3 * (size_t)c.h.N + 1);
   c.dg_colexp.alloc((size_t)cdiv(std::max(c.h.D, c.h.M), kDgGroup) * c.h.N);
   c.dg_redo.alloc((size_t)std::max(c.h.D, c.h.M) * cdiv(c.h.N, 8));
@@ -3944,6 +3972,7 @@ int pqdts_cuda_get_option(pqdts_ctx* c, const char* name, int64_t* value) {
     else if (n == "sched.df_trans") *value = c->df_trans;
     else if (n == "sched.dg_fwd") *value = c->dg_fwd;
     else if (n == "sched.dg_trans") *value = c->dg_trans;
+    else if (n == "sched.dg_bytes") *value = pqdts::dg_held(*c);
     else if (n == "sched.tc_screen") *value = (s.tc && c->tc_ready && c->tc_screen_option != 0) ? 1 : 0;
     else if (n == "graphs.captured") *value = (int64_t)c->graphs.size();
     else throw pqdts::Err(PQDTS_E_ARG, "unknown option " + n);
