@@ -98,6 +98,10 @@ int pqdts_cuda_kernel_launches(pqdts_ctx* ctx, int64_t* count);
  *              effect at the next set_problem.  "df_rows" 0 (default,
  *              chosen by size) / 2 / 4 / 8: band rows per block of those
  *              products (each thread accumulates that many outputs).
+ *   "digit_limit_mb" -1 (default) / 0..2^30: the most device memory, in MB,
+ *              that the digits of "df_products" -1 may take; -1: what is
+ *              free.  Where they do not fit, the products are formed in
+ *              double-FP32.  Takes effect at the next set_problem.
  *   "internal_f" -1 (default) / 0 / 1: where the internal F of
  *              pqdts_cuda_set_problem_coo (nnzF < 0) is computed: -1 on the
  *              device for PQDTS_MIXED problems and on the host for PQDTS_FP64

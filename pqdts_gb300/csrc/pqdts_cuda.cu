@@ -411,6 +411,7 @@ struct pqdts_ctx {
   // F's and F^T's digits, those of X and R (K-major) and their columns'
   // exponents
   bool dg_fwd = false, dg_trans = false;
+  int64_t dg_limit_mb = -1;  // most that their operands may take (-1: what is free)
   pqdts::DgOperand dgF, dgFt;
   pqdts::DBuf<uint16_t> dg_x, dg_r;
   pqdts::DBuf<int> dg_col, dg_colexp;  // k_dg_columns (one more: whether dg_redo marks any)
@@ -1646,9 +1647,34 @@ static int64_t dg_held(const Ctx& c) {
                    c.dg_redo.cap);
 }
 
+// Whether the problem's digits may be laid out: within the limit that the
+// caller gave or, where they take over 4 GB, in what is free beside the
+// line search's probe operands, which are allocated when first used.
+static bool dg_room(const Ctx& c) {
+  const int64_t M = c.h.M, N = c.h.N, D = c.h.D;
+  const auto band = [](const TcOperand& w) {
+    return (int64_t)w.blocks * kTcRows * (2 * kDgSlices * w.kmax + 4 * (w.kmax / kDgGroup + 3));
+  };
+  int64_t need = band(c.tcF) + 2 * kDgSlices * N * c.tc_mp + std::max(M, D) * (N / 8 + 1);
+  if (c.dg_trans) need += band(c.tcFt) + 2 * kDgSlices * N * c.tc_dp;
+  if (c.dg_limit_mb >= 0) return need <= c.dg_limit_mb << 20;
+  if (need < (int64_t)4 << 30) return true;
+  size_t free = 0, total = 0;
+  CK(cudaMemGetInfo(&free, &total));
+  cudaMemPool_t pool;
+  CK(cudaDeviceGetDefaultMemPool(&pool, c.device));
+  uint64_t reserved = 0, used = 0;
+  CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  const int64_t later = 4 * (int64_t)kBatchLS * N * c.tc_mp + ((int64_t)1 << 28);
+  return need + later <= (int64_t)(free + (reserved - used)) + dg_held(c);
+}
+
 // What a problem does not use is given back: the operands are among the largest
-// arrays that a mixed one holds.
+// arrays that a mixed one holds.  Where they do not fit, its products are formed
+// in double-FP32.
 static void setup_dg(Ctx& c) {
+  if (c.dg_fwd && !dg_room(c)) c.dg_fwd = c.dg_trans = false;
   if (!c.dg_trans) {
     c.dgFt.release();
     c.dg_r.release();
@@ -3211,7 +3237,14 @@ static void tune_schedule(Ctx& c, Schedule& s) {
 static void choose_schedule(Ctx& c) {
   const HostProblem& h = c.h;
   setup_tc(c);
-  setup_dg(c);
+  try {
+    setup_dg(c);
+  } catch (const Err& e) {
+    if (!c.dg_fwd || e.code != PQDTS_E_NOMEM) throw;
+    (void)cudaGetLastError();  // another context took the memory meanwhile
+    c.dg_fwd = c.dg_trans = false;
+    setup_dg(c);
+  }
   Schedule s = heuristic_schedule(h);
   if (c.tc_ready) {
     s.tc = 1;
@@ -3903,6 +3936,9 @@ int pqdts_cuda_set_option(pqdts_ctx* c, const char* name, int64_t value) {
     } else if (n == "df_products") {
       if (value < -1 || value > 1) throw pqdts::Err(PQDTS_E_ARG, "df_products must be -1, 0 or 1");
       c->df_option = (int)value;
+    } else if (n == "digit_limit_mb") {
+      if (value < -1 || value > (int64_t)1 << 30) throw pqdts::Err(PQDTS_E_ARG, "digit_limit_mb must be -1..2^30");
+      c->dg_limit_mb = value;
     } else if (n == "internal_f") {
       if (value < -1 || value > 1) throw pqdts::Err(PQDTS_E_ARG, "internal_f must be -1, 0 or 1");
       c->internal_f_option = (int)value;
@@ -3967,6 +4003,7 @@ int pqdts_cuda_get_option(pqdts_ctx* c, const char* name, int64_t* value) {
     else if (n == "tc_wait_ms") *value = (int64_t)(c->tc_wait_ns / 1000000ull);
     else if (n == "tc_wait_probe") *value = c->tc_wait_probe;
     else if (n == "fp64_refine") *value = c->refine_option;
+    else if (n == "digit_limit_mb") *value = c->dg_limit_mb;
     else if (n == "internal_f") *value = c->internal_f_option;
     else if (n == "sched.df_fwd") *value = c->df_fwd;
     else if (n == "sched.df_trans") *value = c->df_trans;

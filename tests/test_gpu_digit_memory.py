@@ -26,3 +26,25 @@ def test_given_back(built, small, precision, option):
         s.set_instance(small, pq.MIXED)
         assert s.get_option("sched.dg_bytes") == held
         assert s.L() == L and (s.dL() == G).all()
+
+
+def test_limit(built, small):
+    """Where the operands may not take their memory, double-FP32 it is, with
+    the bits of df_products = 1; a limit that they meet leaves them in use."""
+    import pqdts_gb300 as pq
+
+    with pq.Solver(0) as s:
+        s.set_option("autotune", 0)
+        s.set_instance(small, pq.MIXED)
+        held = s.get_option("sched.dg_bytes")
+        s.set_option("digit_limit_mb", 0)
+        s.set_instance(small, pq.MIXED)
+        assert s.get_option("sched.dg_fwd") == 0 and s.get_option("sched.dg_bytes") == 0
+        L, G = s.L(), s.dL()
+        s.set_option("df_products", 1)
+        s.set_instance(small, pq.MIXED)
+        assert s.L() == L and (s.dL() == G).all()
+        s.set_option("df_products", -1)
+        s.set_option("digit_limit_mb", held // 2**20 + 1)
+        s.set_instance(small, pq.MIXED)
+        assert s.get_option("sched.dg_fwd") == 1 and s.get_option("sched.dg_bytes") == held
