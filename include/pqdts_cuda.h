@@ -114,10 +114,9 @@ int pqdts_cuda_kernel_launches(pqdts_ctx* ctx, int64_t* count);
  *              decrease; 1 for every stage-2 iteration.
  *   "tc_wait_ms" 2000 (default) / 1..60000: limit of each barrier wait in
  *              the tensor-core kernels; a wait that runs out makes the call
- *              fail with PQDTS_E_CUDA ("a barrier wait timed out"), nothing
- *              having been written to the caller's arrays by L, dL and BF32
- *              and the kernel's tensor memory freed, and the context stays
- *              usable (its X after a solve that failed so is undefined).
+ *              fail with PQDTS_E_CUDA ("a barrier wait timed out"), the
+ *              kernel's tensor memory freed; what the call was to write is
+ *              undefined (after a solve: X too), and the context stays usable.
  *   "tc_wait_probe" 0 (default) / 1: test hook of that error path -- each
  *              kernel's copy producer first waits on a barrier that nothing
  *              arrives on, so the wait runs out before any copy or MMA.
