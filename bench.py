@@ -12,7 +12,8 @@ One "step" = one full solve.
     `config.parity`), so the CPU baseline does exactly the same iterations
     and reaches exactly the same objective L64.
   mixed (reported beside it): tensor-core (split-BF16x3) Hessian products /
-    FP32 CG, gradient and objective checks in double-FP32 (~1e-13 relative),
+    FP32 CG, gradient and objective checks by exact digits on the tensor cores
+    and in double-FP32 (~1e-13 relative),
     FP64 line-search decisions and projection, run until its objective is
     within 1e-8 relative of L64 (an extra stopping rule, off by default).
 `value` = seconds per solve with the problem resident in HBM (CUDA events on
@@ -633,9 +634,9 @@ def run_ours(args):
                        "rel_obj_vs_L64": (ms[-1]["L"] - L64) / L64, "reached": ms[-1]["L"] <= target,
                        "outer": ms[-1]["outer"], "cg": ms[-1]["cg"], "refine": ms[-1]["refine"],
                        "tensor_cores": bool(sm.get_option("sched.tc")),
-                       "double_fp32_gradient_and_checks": bool(sm.get_option("sched.df_trans")),
+                       "digit_gradient_and_checks": bool(sm.get_option("sched.dg_trans")),
                        # GPU time per solve in the objective (L: checks of the chosen
-                       # steps) and gradient (dL) regions, double-FP32 products included
+                       # steps) and gradient (dL) regions, their products included
                        # (the region timers' solve)
                        "L_region_s_per_solve": l1[0] - l0[0],
                        "dL_region_s_per_solve": g1[0] - g0[0],
@@ -887,7 +888,7 @@ def run_workload(name, args):
                 tl, tg = s.timer("L"), s.timer("dL")
                 out[tag] = {"seconds": el, "outer": st["outer"], "cg": st["cg"],
                             "L_seconds": tl[0], "L_calls": tl[1], "dL_seconds": tg[0], "dL_calls": tg[1],
-                            "double_fp32": bool(s.get_option("sched.df_fwd")) if prec == pq.MIXED else False,
+                            "digits": bool(s.get_option("sched.dg_fwd")) if prec == pq.MIXED else False,
                             "s_per_outer": el / max(1, st["outer"]), "L": st["L"],
                             "tensor_cores": bool(s.get_option("sched.tc")) if prec == pq.MIXED else False,
                             "bf_seconds": bf[0], "bf_calls": bf[1],
