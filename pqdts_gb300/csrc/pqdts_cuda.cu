@@ -50,7 +50,8 @@ constexpr int kMaxLS = 100;                // do i = 1, 100 (374, 420, 466)
 constexpr int kBatchLS = 8;                // step lengths evaluated per sweep
 constexpr int64_t kPinnedRows = 4096;       // simplexproj calls of up to this many values go through pinned memory
 constexpr int64_t kProjKeep = 1 << 25;      // ... and of up to this many keep their device rows for the next one
-constexpr int kElemGrid = 152 * 8;         // elementwise grids: 8 blocks per SM
+constexpr int kSMs = 152;                  // of a GB300
+constexpr int kElemGrid = kSMs * 8;         // elementwise grids: 8 blocks per SM
 constexpr size_t kRowSmemMax = 200u * 1024u;  // k_simplex_smem's rows staged in shared memory up to this size
 
 struct Err : std::runtime_error {
@@ -654,7 +655,7 @@ static bool tc_wanted(const Ctx& c) {
 
 // About eight blocks an SM for nb tiles, up to 16 a tile.
 static dim3 tile_build_grid(int64_t nb) {
-  return dim3((unsigned)nb, (unsigned)std::max<int64_t>(1, std::min<int64_t>(16, 8 * 152 / nb)));
+  return dim3((unsigned)nb, (unsigned)std::max<int64_t>(1, std::min<int64_t>(16, 8 * kSMs / nb)));
 }
 
 // The problem's arrays on the device (maxr_state: the seeded stream before
@@ -899,7 +900,7 @@ static void need_problem(Ctx& c) {
 // ---------------------------------------------------------------------------
 static void rebuild(Ctx& c, double* X, const double* saved, int32_t* chg) {
   const int M = (int)c.h.M, N = (int)c.h.N;
-  k_rebuild_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(X, (int64_t)M * N, c.maxr.p, M, N, saved, chg);
+  k_rebuild_t<<<cdiv(M, 32), kTileThreads, 0, c.st>>>(X, c.maxr.p, M, N, saved, chg);
   post_launch(c);
 }
 
@@ -916,7 +917,7 @@ static void launch_colchain(Ctx& c, const double* a, const double* b, int64_t st
   const int M = (int)c.h.M, N = (int)c.h.N;
   const int chains = N * (OP == 2 ? 2 : 1);
   double* sc = advance ? c.sc.p : nullptr;
-  if (M >= (OP == 2 ? 1500 : 500) && (int64_t)chains * B <= (OP == 2 ? 3 : 2) * 152) {
+  if (M >= (OP == 2 ? 1500 : 500) && (int64_t)chains * B <= (OP == 2 ? 3 : 2) * kSMs) {
     k_colchain_b<OP><<<dim3(chains, B), 32 * kBcWarps, 0, c.st>>>(a, b, stride, M, N, c.h.gam, out, out2, pred, sum_out,
                                                                   ostride, counter, sc, c.cglog.p, kMaxCG);
   } else {
@@ -982,7 +983,7 @@ static int rows_per_block(int N) {
 
 // Whether a column product of `warps` warps has so few (at most four an SM
 // sub-partition) that each is better fed by another (fed_chain).
-static bool few_warps(int64_t warps) { return warps <= 4 * 4 * 152; }
+static bool few_warps(int64_t warps) { return warps <= 4 * 4 * kSMs; }
 
 // F.X (B stacked inputs, xstride apart) with the epilogue MODE of k_fwd, in
 // the context's form: column-tiled, or row-flattened (rows = 1; the same
@@ -1009,7 +1010,7 @@ static void launch_fwd(Ctx& c, const T* fv, const T* X, int64_t xstride, const d
             M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride, c.xcmask.p, c.xccnt.p,
             c.xclist.p, P, R, pred, count, cols);
       else
-        k_fwd_col<T, MODE><<<dim3(cdiv(N, kTcWarps), tiles, B), dim3(32, kTcWarps), 0, c.st>>>(
+        k_fwd_col<MODE><<<dim3(cdiv(N, kTcWarps), tiles, B), dim3(32, kTcWarps), 0, c.st>>>(
             M, N, D, c.fwtile.p, c.fwtile_lo.p, c.fwtile_hi.p, c.fwtile_off.p, X, xstride, c.xcmask.p, c.xccnt.p,
             c.xclist.p, P, R, pred, count, cols);
       post_launch(c);
@@ -1270,7 +1271,7 @@ static void launch_trans_shape(Ctx& c, TransShape sh, const T* tv, const T* R, c
             M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, acc, pred,
             count, ik, reduced ? c.maxr.p : nullptr, cols);
       else
-        k_trans_col<T><<<dim3(cdiv(N, kTcWarps), tiles), dim3(32, kTcWarps), 0, c.st>>>(
+        k_trans_col<<<dim3(cdiv(N, kTcWarps), tiles), dim3(32, kTcWarps), 0, c.st>>>(
             M, N, D, c.ftile.p, c.ftile_lo.p, c.ftile_hi.p, c.ftile_off.p, R, c.rmask.p, c.ccnt.p, c.clist.p, acc, pred,
             count, ik, reduced ? c.maxr.p : nullptr, cols);
       post_launch(c);
@@ -2200,10 +2201,10 @@ static void cg_solve(Ctx& c, CGBufs<T>& b, const T* fv, const T* tv, double bdfa
 }
 
 // k_condat over B stacked sets of M rows: one row a warp until every SM
-// sub-partition of the GPU (152 SMs x 4) has a warp, then more rows a warp.
+// sub-partition of the GPU has a warp, then more rows a warp.
 static void launch_condat(const double* X, const double* S, const double* alphas, double* out, double* aux,
                           int64_t stride, int M, int N, int B, cudaStream_t st) {
-  const int RP = (int)std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)M * B + 607) / 608));
+  const int RP = (int)std::max<int64_t>(1, std::min<int64_t>(32, ((int64_t)M * B + 4 * kSMs - 1) / (4 * kSMs)));
   k_condat<<<dim3(cdiv(M, RP * kCondatWarps), B), 32 * kCondatWarps, 0, st>>>(X, S, alphas, out, aux, stride, M, N,
                                                                               RP);
 }
