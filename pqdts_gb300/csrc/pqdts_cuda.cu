@@ -310,6 +310,7 @@ struct DgOperand {
   TcSched sched;
   int bn = 0, stages = 0;
   int groups = 0;     // of K that a row block's window meets, at most
+  bool redo64 = false;  // what is left is formed in FP64 (k_dg_redo)
   int fine = 0;       // bits of the sums below 2^-48 of the scales
   float floor = 0.f;  // sum of magnitudes below which an output is formed again
   void release() {
@@ -1093,6 +1094,13 @@ static void fwd_df(Ctx& c, const double* X, double* R) {
     dg_split(c, X, (int)c.h.M, c.tc_mp, c.dg_x);
     redo = dg_product<MODE>(c, c.dgF, c.tcF, (int)c.h.D, X, R, nullptr, nullptr, 0.0);
   }
+  if (c.dg_fwd && c.dgF.redo64) {
+    const int D = (int)c.h.D;
+    k_dg_redo<MODE><<<D * cdiv(c.h.N, 32), 32 * kDgRedoWarps, 0, c.st>>>(bands_of(c), c.fval.p, X, c.P.p, nullptr, 0.0,
+                                                                         R, nullptr, redo);
+    post_launch(c);
+    return;
+  }
   require(c.xdf.p, "xdf");
   k_split_df<<<elem_grid(MN), 256, 0, c.st>>>(X, MN, 1.0, c.xdf.p, redo.any);
   post_launch(c);
@@ -1345,16 +1353,22 @@ static void op_dL(Ctx& c) {
       dg_split(c, c.R.p, D, c.tc_dp, c.dg_r);
       redo = dg_product<4>(c, c.dgFt, c.tcFt, M, c.R.p, c.Gf.p, g, c.X.p, c2g);
     }
-    k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p, redo.any);
-    post_launch(c);
-    const int rb = df_rows_per_block(M, N, c.df_rows, c.num_sms, redo.bits != nullptr);
-    const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
-    const dim3 grid(cdiv(M, rb), cdiv(N, threads));
-    DevBands bd = bands_of(c);
-    if (rb == 8) k_trans_df<8><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
-    else if (rb == 4) k_trans_df<4><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
-    else k_trans_df<2><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
-    post_launch(c);
+    if (c.dg_trans && c.dgFt.redo64) {
+      k_dg_redo<4><<<M * cdiv(N, 32), 32 * kDgRedoWarps, 0, c.st>>>(bands_of(c), c.tval.p, c.R.p, nullptr, c.X.p, c2g,
+                                                                   c.Gf.p, g, redo);
+      post_launch(c);
+    } else {
+      k_split_df<<<elem_grid((int64_t)D * N), 256, 0, c.st>>>(c.R.p, (int64_t)D * N, 1.0, c.rdf.p, redo.any);
+      post_launch(c);
+      const int rb = df_rows_per_block(M, N, c.df_rows, c.num_sms, redo.bits != nullptr);
+      const int threads = 32 * std::min(kDfColWarps, cdiv(N, 32));
+      const dim3 grid(cdiv(M, rb), cdiv(N, threads));
+      DevBands bd = bands_of(c);
+      if (rb == 8) k_trans_df<8><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
+      else if (rb == 4) k_trans_df<4><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
+      else k_trans_df<2><<<grid, threads, 0, c.st>>>(bd, c.tdf.p, c.rdf.p, c.X.p, c2g, g, c.Gf.p, redo);
+      post_launch(c);
+    }
     if (!c.fullspace) {
       k_reduced_from_full<<<M, std::min(256, std::max(32, cdiv(N, 32) * 32)), 0, c.st>>>(c.Gf.p, c.maxr.p, N, c.G.p);
       post_launch(c);
@@ -1597,6 +1611,11 @@ static void setup_digits(Ctx& c, DgOperand& op, TcOperand& win, bool trans, DBuf
   const int terms = widths.empty() ? 0 : *std::max_element(widths.begin(), widths.end());
   op.fine = dg_fine(terms);
   op.groups = win.kmax / kDgGroup + 2;
+  // k_dg_redo with every output left would hold the FP64 pipe for ~40 us (64
+  // cycles a warp and term on 4 x 152 sub-partitions).  set_x, L and dL at a late
+  // iterate, M = 200 / 300 / 500: 177 / 205 / 243 us (double-FP32 for what is left
+  // 231 / 260 / 315, for everything 171 / 196 / 249).
+  op.redo64 = (int64_t)(trans ? c.h.M : c.h.D) * cdiv(N, 32) * terms <= 800000;
   op.floor = dg_floor(terms, op.groups, op.fine);
   op.dig.alloc((size_t)S * rows * win.kmax);
   op.rowexp.alloc((size_t)rows * op.groups);

@@ -664,4 +664,64 @@ __global__ void __launch_bounds__(kDgThreads, 1)
   }
 }
 
+// The outputs that a digit product left (redo), in FP64: a block per row and 32
+// columns, lane = column, the row's band in kDgRedoWarps shares of one warp each
+// (a row at a time in one warp took twice as long, bound by its loads); out,
+// out2, P, V and the modes as k_dg_band_product's.  For products so small that
+// the double-FP32 kernels' launches (splitting the operand, masks, product) and
+// latencies are what they cost.
+constexpr int kDgRedoWarps = 4;
+template <int MODE>
+__global__ void __launch_bounds__(32 * kDgRedoWarps)
+    k_dg_redo(DevBands f, const double* __restrict__ val, const double* __restrict__ B, const double* __restrict__ P,
+              const double* __restrict__ V, double c2gam, double* out, double* out2, DfRedo redo) {
+  if (*redo.any == 0) return;
+  __shared__ double part[kDgRedoWarps][32];
+  const int N = f.N, R = MODE == 4 ? f.M : f.D, ng = (N + 31) >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = blockIdx.x / ng, n = (blockIdx.x % ng) * 32 + lane;
+  const bool need = n < N && ((redo.bits[(int64_t)r * redo.pitch + (n >> 3)] >> (n & 7)) & 1);
+  if (!__any_sync(0xffffffffu, need)) return;  // the same in every warp
+  int lo, w;
+  int64_t off;
+  dg_row<MODE == 4>(f, r, lo, w, off);
+  const int k0 = (int)((int64_t)w * warp / kDgRedoWarps), k1 = (int)((int64_t)w * (warp + 1) / kDgRedoWarps);
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  if (need) {
+    const double* a = val + off;
+    const double* b = B + (int64_t)lo * N + n;
+    int k = k0;
+    for (; k + 8 <= k1; k += 8) {
+      double x[8], y[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        x[q] = a[k + q];
+        y[q] = b[(int64_t)(k + q) * N];
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) s[q & 3] = fma(x[q], y[q], s[q & 3]);
+    }
+    for (; k < k1; ++k) s[0] = fma(a[k], b[(int64_t)k * N], s[0]);
+  }
+  part[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+  __syncthreads();
+  if (warp > 0 || !need) return;
+  double v = part[0][lane];
+#pragma unroll
+  for (int q = 1; q < kDgRedoWarps; ++q) v += part[q][lane];
+  const int64_t o = (int64_t)r * N + n;
+  if (MODE != 4) {
+    v -= P[o];
+    out[o] = MODE == 0 ? 2.0 * v : v;
+    return;
+  }
+  if (c2gam != 0.0) {
+    const double vi = V[o];
+    if (r < R - 1) v = fma(c2gam, vi - V[o + N], v);
+    if (r > 0) v = fma(-c2gam, V[o - N] - vi, v);
+  }
+  if (out) out[o] = v;
+  if (out2) out2[o] = v;
+}
+
 }  // namespace pqdts
